@@ -86,7 +86,7 @@ using namespace mkf;
 
 MKF_API int mkfFieldBPFD(uint64_t *pBPFD, const MKFFieldDesc *pF, const MKFThreshSet *pT, int flags, void *stream)
 {
-   return fieldBPFD(pBPFD, pF, pT, flags, (cudaStream_t)stream, nullptr);
+   return fieldBPFD(pBPFD, pF, pT, flags, (cudaStream_t)stream);
 }
 
 MKF_API int mkfFieldBPFDMoments(uint64_t *pBPFD, double *pMom, const MKFFieldDesc *pF, const MKFThreshSet *pT,
@@ -104,25 +104,14 @@ MKF_API int mkfFieldBPFDMoments(uint64_t *pBPFD, double *pMom, const MKFFieldDes
       if (e == cudaSuccess) { e = cudaMemsetAsync(pMom, 0, (size_t)K * 4 * sizeof(double), s); }
       if (e != cudaSuccess) { return cudaFail(e, "cudaMemsetAsync"); }
    }
-   FusedArgs a;
-   memset(&a, 0, sizeof(a));
-   a.f = pF->p;
-   const bool planar = !(pF->stride[0] | pF->stride[1] | pF->stride[2]);
-   a.sx = planar ? 1 : pF->stride[0];
-   a.sy = planar ? (int64_t)X : pF->stride[1];
-   a.sz = planar ? (int64_t)X * Y : pF->stride[2];
-   a.X = X; a.Y = Y; a.Z = Z;
-   a.K = K;
-   a.out = pBPFD;
-   uint32_t masks[2];
-   for (int k = 0; k < K; k++) {
-      const double t = pT->t[k];
-      if (pF->enc == ENC_F32) { floatBoundsPlain(t, a.tlo[k], a.thi[k]); }
-      else { a.tlo[k] = a.thi[k] = t; }
-      a.outRow[k] = k;
-      masks[k] = (pT->m ? pT->m[k] : pT->mAll) & BMC_AL;
-   }
-   return launchWordsMoments(a, pF->enc, masks, pMom, s);
+   ThreshSplit q;  // every threshold in order, constant maps included (their tests all fail or hold)
+   q.n = K;
+   for (int k = 0; k < K; k++) { q.idx[k] = k; }
+   WordTask w;
+   fillWordTask(w, pF, pT, q, 0, K, 0);
+   w.out = pBPFD;
+   w.mom = pMom;
+   return launchWordsMoments(w, pF->enc, s);
 }
 
 // ---------------------------------------------------------------- batches
@@ -155,7 +144,6 @@ struct MKFBatchPlan
    cudaGraphExec_t graphExec = nullptr;
 };
 
-static constexpr int kChunkItems = 64;
 static constexpr int kPlanCounters = 2 + 2 * kThVariants;
 
 static void freePlan(MKFBatchPlan *p)
@@ -202,18 +190,10 @@ static int createPlan(MKFBatchPlan **pp, uint64_t *pBPFD, const MKFFieldDesc *pF
       for (size_t c = c0; c < p->consts.size(); c++) { p->constCells.push_back(cells); }
       if (cells > 0 && kind == kPlanWords) {
          const int e = d->enc == ENC_F32 ? 0 : 1;
-         const int f = (int)wtasks[e].size();
-         for (long long b = 0; b < w.nItems; b += kChunkItems) {
-            wchunks[e].push_back({f, 0, b, std::min<long long>(b + kChunkItems, w.nItems)});
-         }
          w.out = pBPFD;
          wtasks[e].push_back(w);
       } else if (cells > 0 && kind == kPlanThermo) {
          const int e = d->enc == ENC_F32 ? 0 : 1;
-         const int f = (int)tasks[e].size();
-         for (long long b = 0; b < t.nItems; b += kChunkItems) {
-            chunks[e].push_back({f, 0, b, std::min<long long>(b + kChunkItems, t.nItems)});
-         }
          t.out = pBPFD;
          tasks[e].push_back(t);
       } else if (cells > 0 && varying) {
@@ -235,6 +215,7 @@ static int createPlan(MKFBatchPlan **pp, uint64_t *pBPFD, const MKFFieldDesc *pF
    cudaError_t e = cudaMalloc(&p->dCounter, kPlanCounters * sizeof(unsigned));
    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
       if (tasks[k].empty()) { continue; }
+      chunks[k] = thermoChunks(tasks[k]);
       p->groups[k] = groupThermoChunks(chunks[k], tasks[k]);
       e = cudaMalloc(&p->dTasks[k], tasks[k].size() * sizeof(FieldTask));
       if (e == cudaSuccess) { e = cudaMalloc(&p->dChunks[k], chunks[k].size() * sizeof(BatchChunk)); }
@@ -244,6 +225,7 @@ static int createPlan(MKFBatchPlan **pp, uint64_t *pBPFD, const MKFFieldDesc *pF
    }
    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
       if (wtasks[k].empty()) { continue; }
+      wchunks[k] = wordChunks(wtasks[k]);
       e = cudaMalloc(&p->dWTasks[k], wtasks[k].size() * sizeof(WordTask));
       if (e == cudaSuccess) { e = cudaMalloc(&p->dWChunks[k], wchunks[k].size() * sizeof(BatchChunk)); }
       if (e == cudaSuccess) { e = cudaMemcpy(p->dWTasks[k], wtasks[k].data(), wtasks[k].size() * sizeof(WordTask), cudaMemcpyHostToDevice); }
@@ -292,7 +274,7 @@ static int planLaunchOn(MKFBatchPlan *p, cudaStream_t s)
       ts.t = fb.t.data();
       ts.m = fb.perThreshold ? fb.m.data() : nullptr;
       ts.mAll = fb.mAll;
-      rc = fieldBPFD(p->out + fb.rowBase * 256, &fb.d, &ts, MKF_F_ACCUMULATE, s, nullptr);
+      rc = fieldBPFD(p->out + fb.rowBase * 256, &fb.d, &ts, MKF_F_ACCUMULATE, s);
    }
    return rc;
 }
@@ -456,7 +438,7 @@ MKF_API int mkfFieldBPFDHost(uint64_t *pBPFDH, const MKFFieldDesc *pF, const MKF
       MKFFieldDesc sub = *pF;
       sub.p = gHost.stage[b];
       sub.def[2] = (int32_t)nPl;
-      rc = fieldBPFD(gHost.counts, &sub, pT, MKF_F_ACCUMULATE, gHost.comp, nullptr);
+      rc = fieldBPFD(gHost.counts, &sub, pT, MKF_F_ACCUMULATE, gHost.comp);
       cudaEventRecord(gHost.consumed[b], gHost.comp);
    }
    if (rc == MKF_OK) {

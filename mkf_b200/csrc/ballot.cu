@@ -1,0 +1,242 @@
+// ballot.cu - fused counting kernel for one threshold on fields of middle size: map words packed by
+// warp votes from registers.
+//
+// The other kernel for few thresholds (words.cuh) lets each lane pack its own row from a copy of the
+// tile in shared memory. That costs fewer instructions per threshold, but a FP64 tile row holds only
+// 16 elements there, and its larger CTAs start more slowly; the rule at useBallots has the figures.
+// A warp item is a tile of 32 x positions (31 cells), 32 rows (31 row pairs) and D planes, walked plane
+// by plane:
+//  * load: lane = x; the warp issues the 32 rows' coalesced loads at once;
+//  * pack: one ballot per row gives that row's 32-bit map word; lane r keeps row r's;
+//  * count: lane = row pair. A cell's eight corners are bits b and b+1 of four words (this lane's
+//    row and the next lane's row, previous and current plane), so all-ones and all-zeros cells
+//    are popcounts of ANDs and ORs of the words and their one-bit shifts; only mixed cells form
+//    their 8-bit code, counted in a per-CTA shared histogram.
+#include <cmath>
+#include <cstring>
+#include "fused.cuh"
+
+namespace mkf {
+
+// FP32 fields whose items lie inside the field and are at least kBlPfDepth planes deep load the next
+// plane while counting the current one (two plane buffers in registers at 2 CTAs per SM, 128
+// registers): 1.55 x faster on a 1024^3 FP32 GRF (0.70 vs 1.09 ms), slower for shallow items, which
+// keep the single buffer at 4 CTAs per SM.
+static constexpr int kBlPfDepth = 16;
+static constexpr int kBlWarps = 8;
+static constexpr int kBlD = 32;  // default planes of cells per work item
+// Untuned fields get at least this many work items per SM (the slab depth is halved until they
+// do): measured on 256^3 to 512^3 fields, fewer items than ~0.6 of the resident warps leave SMs
+// idle while deeper items win nothing.
+static constexpr int kBlItemsPerSM = 20;
+
+// The map bit of the tests in MODE (WordTask::mode): 1 f > tlo, 2 f < thi, 3 either.
+template <int MODE, typename T>
+__device__ __forceinline__ bool ballotBit(T v, T tlo, T thi)
+{
+   return (MODE == 1 && v > tlo) || (MODE == 2 && v < thi) || (MODE == 3 && (v > tlo || v < thi));
+}
+
+// State of one warp item between planes: the previous plane's map words and the cell counts.
+struct BallotCarry
+{
+   uint32_t pw = 0, pn = 0;  // previous plane: this lane's row word and the next row's
+   uint32_t n0 = 0, n1 = 0;  // all-zeros and all-ones cells counted by this lane
+};
+
+// Load one plane's 32 x 32 tile (lane = x). INNER: every row of the tile lies inside the field
+// and the row stride in bytes `syb` times 31 fits 32 bits, so each row address is one multiply-add
+// on the plane pointer; otherwise rows past the field end repeat its last row (their cells are
+// masked out when counted) and addresses are formed in 64 bits.
+template <typename T, bool INNER>
+__device__ __forceinline__ void loadPlane(T (&v)[32], const T *__restrict__ p, int64_t sy, uint32_t syb, int nRow)
+{
+#pragma unroll
+   for (int r = 0; r < 32; r++) {
+      if (INNER) {
+         v[r] = __ldg((const T *)((const char *)p + (uint64_t)(syb * (uint32_t)r)));
+      } else {
+         v[r] = __ldg(p + (int64_t)min(r, nRow - 1) * sy);
+      }
+   }
+}
+
+// Map, pack and count one plane (see the file comment). `first`: no previous plane yet.
+// `sRow` is the warp's 32-word transposition buffer.
+template <int MODE, typename T>
+__device__ __forceinline__ void countPlane(const T (&v)[32], BallotCarry &c, T tlo, T thi, bool xin, int lane, uint32_t vm, bool first,
+                                           uint32_t *sRow, uint32_t *sHist)
+{
+#pragma unroll
+   for (int r = 0; r < 32; r++) {
+      // every lane stores the same (warp-uniform) word
+      sRow[r] = __ballot_sync(FULL, xin && ballotBit<MODE>(v[r], tlo, thi));
+   }
+   __syncwarp();
+   const uint32_t cw = sRow[lane];
+   __syncwarp();
+   const uint32_t cn = __shfl_down_sync(FULL, cw, 1);
+   if (!first) {
+      const uint32_t a0 = c.pw, a1 = c.pn, a2 = cw, a3 = cn;
+      const uint32_t all = a0 & (a0 >> 1) & a1 & (a1 >> 1) & a2 & (a2 >> 1) & a3 & (a3 >> 1) & vm;
+      const uint32_t any = a0 | (a0 >> 1) | a1 | (a1 >> 1) | a2 | (a2 >> 1) | a3 | (a3 >> 1);
+      c.n1 += __popc(all);
+      c.n0 += __popc(vm & ~any);
+      uint32_t mixed = vm & any & ~all;
+      if (mixed) {
+         // word j's bits b, b+1 go to code bits 2j, 2j+1: pre-shift j's word left by 2j as a
+         // 64-bit (hi:lo) pair, so one funnel shift by b brings them into place
+         const uint32_t l1 = a1 << 2, h1 = a1 >> 30, l2 = a2 << 4, h2 = a2 >> 28, l3 = a3 << 6, h3 = a3 >> 26;
+         do {
+            const int b = 31 - __clz(mixed);
+            mixed ^= 1u << b;
+            uint32_t code = (__funnelshift_r(l1, h1, b) & ~3u) | ((a0 >> b) & 3u);
+            code = (__funnelshift_r(l2, h2, b) & ~15u) | (code & 15u);
+            code = (__funnelshift_r(l3, h3, b) & ~63u) | (code & 63u);
+            atomicAdd(sHist + (code & 255u), 1u);
+         } while (mixed);
+      }
+   }
+   c.pw = cw;
+   c.pn = cn;
+}
+
+// One warp counts work item `it` (31 x 31 cells, D planes) of field `a` into the CTA's histogram
+// and all-zeros / all-ones totals. INNER: the field is at least 32 x 32 in x and y with a positive
+// row stride below 2^32 / 31 bytes; edge tiles are then shifted back inside the field (their cells
+// already counted by the neighbouring tile are masked out), so no load needs clamping.
+// PF: the next plane's loads are issued before the current plane is counted (two plane buffers
+// in registers, alternating; INNER fields only).
+template <typename T, int MODE, bool INNER, bool PF>
+__device__ __forceinline__ void ballotItem(const WordTask &a, long long it, T tlo, T thi, uint32_t *sRow, uint32_t *sHist,
+                                           unsigned long long *sEnds)
+{
+   const int lane = threadIdx.x & 31;
+   const T *__restrict__ F = (const T *)a.f;
+   const uint32_t syb = (uint32_t)(a.sy * (int64_t)sizeof(T));
+   const int ix = (int)(it % a.nStripX);
+   const long long rest = it / a.nStripX;
+   const int iy = (int)(rest % a.nTileY);
+   const int iz = (int)(rest / a.nTileY);
+   // this item's cells: x in [xs, xe), y in [ys, ye), z in [z0, z0 + nPln)
+   const int xs = 31 * ix, ys = 31 * iy, z0 = a.D * iz;
+   const int xe = min(xs + 31, a.X - 1), ye = min(ys + 31, a.Y - 1);
+   const int nPln = min(a.D, a.Z - 1 - z0);
+   // tile origin: bit b of a word is x0 + b, lane l counts the row pair y0 + l
+   const int x0 = INNER ? min(xs, a.X - 32) : xs;
+   const int y0 = INNER ? min(ys, a.Y - 32) : ys;
+   const int nRow = INNER ? 32 : min(32, a.Y - y0);
+   const bool xin = INNER || x0 + lane < a.X;
+   const T *base = F + (long long)(INNER ? x0 + lane : min(x0 + lane, a.X - 1)) * a.sx + (long long)y0 * a.sy +
+                   (long long)z0 * a.sz;
+   const uint32_t vm = (y0 + lane >= ys && y0 + lane < ye)
+                          ? ((0xFFFFFFFFu >> (32 - (xe - x0))) & (0xFFFFFFFFu << (xs - x0)))
+                          : 0u;
+   BallotCarry c;
+   if (PF && INNER) {
+      T va[32], vb[32];
+      loadPlane<T, INNER>(va, base, a.sy, syb, nRow);
+      for (int p = 0; p <= nPln; p += 2) {
+         if (p + 1 <= nPln) { loadPlane<T, INNER>(vb, base + (long long)(p + 1) * a.sz, a.sy, syb, nRow); }
+         countPlane<MODE>(va, c, tlo, thi, xin, lane, vm, p == 0, sRow, sHist);
+         if (p + 1 > nPln) { break; }
+         if (p + 2 <= nPln) { loadPlane<T, INNER>(va, base + (long long)(p + 2) * a.sz, a.sy, syb, nRow); }
+         countPlane<MODE>(vb, c, tlo, thi, xin, lane, vm, false, sRow, sHist);
+      }
+   } else {
+      for (int p = 0; p <= nPln; ++p) {
+         T v[32];
+         loadPlane<T, INNER>(v, base + (long long)p * a.sz, a.sy, syb, nRow);
+         countPlane<MODE>(v, c, tlo, thi, xin, lane, vm, p == 0, sRow, sHist);
+      }
+   }
+   const unsigned long long s0 = __reduce_add_sync(FULL, c.n0);
+   const unsigned long long s1 = __reduce_add_sync(FULL, c.n1);
+   if (lane == 0) {
+      if (s0) { atomicAdd(&sEnds[0], s0); }
+      if (s1) { atomicAdd(&sEnds[1], s1); }
+   }
+}
+
+template <typename T, int MODE, bool INNER, int MINB, bool PF>
+__global__ void __launch_bounds__(kBlWarps * 32, MINB) ballotBPFD(const __grid_constant__ WordTask a)
+{
+   __shared__ uint32_t sHist[256];
+   __shared__ unsigned long long sEnds[2];  // all-zeros, all-ones cells
+   __shared__ uint32_t sRows[kBlWarps][32];
+   for (int i = threadIdx.x; i < 256; i += blockDim.x) { sHist[i] = 0; }
+   if (threadIdx.x < 2) { sEnds[threadIdx.x] = 0; }
+   __syncthreads();
+   const T tlo = (T)a.tlo[0], thi = (T)a.thi[0];
+   const long long gw = (long long)blockIdx.x * kBlWarps + (threadIdx.x >> 5);
+   const long long nw = (long long)gridDim.x * kBlWarps;
+   for (long long it = gw; it < a.nItems; it += nw) {
+      ballotItem<T, MODE, INNER, PF>(a, it, tlo, thi, sRows[threadIdx.x >> 5], sHist, sEnds);
+   }
+   __syncthreads();
+   // mixed codes as counted, 0 / 255 from the totals; counted negated, code c belongs in bin 255 - c
+   for (int c = threadIdx.x; c < 256; c += blockDim.x) {
+      unsigned long long v = sHist[c];
+      if (c == 0) { v += sEnds[0]; }
+      if (c == 255) { v += sEnds[1]; }
+      if (v) { atomicAdd((unsigned long long *)(a.out + (size_t)a.outRow[0] * 256 + ((a.inv & 1u) ? 255 - c : c)), v); }
+   }
+}
+
+template <typename T, int MODE, bool INNER, int MINB, bool PF>
+static int launchBallotT(const WordTask &a, cudaStream_t s)
+{
+   static std::atomic<int> occ{0};
+   auto kern = ballotBPFD<T, MODE, INNER, MINB, PF>;
+   const int blocksPerSM = cachedOccupancy(occ, kern, kBlWarps * 32, 0);
+   long long grid = (a.nItems + kBlWarps - 1) / kBlWarps;
+   const long long cap = (long long)smCount() * blocksPerSM;
+   if (grid > cap) { grid = cap; }
+   if (grid < 1) { grid = 1; }
+   kern<<<(unsigned)grid, kBlWarps * 32, 0, s>>>(a);
+   return cudaFail(cudaGetLastError(), "ballotBPFD launch");
+}
+
+template <typename T, int MODE>
+static int launchBallotM(const WordTask &a, cudaStream_t s)
+{
+   const int64_t syb = a.sy * (int64_t)sizeof(T);
+   const bool inner = a.X >= 32 && a.Y >= 32 && syb > 0 && syb * 31 < (int64_t)1 << 32;
+   constexpr bool F32 = sizeof(T) == 4;
+   if (!inner) { return launchBallotT<T, MODE, false, 2, false>(a, s); }
+   if (F32 && a.D >= kBlPfDepth) { return launchBallotT<T, MODE, true, 2, F32>(a, s); }
+   return launchBallotT<T, MODE, true, F32 ? 4 : 2, false>(a, s);
+}
+
+template <typename T>
+static int dispatchBallot(const WordTask &a, cudaStream_t s)
+{
+   switch (a.mode[0]) {
+      case 1: return launchBallotM<T, 1>(a, s);
+      case 2: return launchBallotM<T, 2>(a, s);
+      default: return launchBallotM<T, 3>(a, s);
+   }
+}
+
+// B200, device time of a call, this kernel against the other (words.cuh): FP32 64^3 7.9 / 6.9 us,
+// 128^3 8.3 / 8.9, 256^3 18.8 / 20.2, 301 x 333 x 277 33.7 / 34.6, 512^3 115 / 109,
+// 128 x 2048 x 2048 398 / 359; FP64 64^3 8.0 / 6.1, 128^3 9.2 / 9.6, 256 x 512 x 512 86 / 97,
+// 333 x 401 x 487 85 / 111. With two thresholds the other is faster from 512^3 on and in small fields.
+bool useBallots(const WordTask &a, int enc)
+{
+   const double voxels = (double)a.X * a.Y * a.Z;
+   return a.K == 1 && voxels >= (double)(1 << 20) && (enc == ENC_F64 || voxels < (double)(1 << 26));
+}
+
+int launchBallots(WordTask &a, int enc, cudaStream_t s)
+{
+   a.nStripX = (a.X - 1 + 30) / 31;
+   a.nTileY = (a.Y - 1 + 30) / 31;
+   a.D = tunedDepth(kFamWords, enc, a.K, a.X, a.Y, a.Z,
+                    sizeDepth(kBlD, (long long)a.nStripX * a.nTileY, a.Z, (long long)smCount() * kBlItemsPerSM));
+   a.nSlabZ = (a.Z - 1 + a.D - 1) / a.D;
+   a.nItems = (long long)a.nStripX * a.nTileY * a.nSlabZ;
+   return enc == ENC_F32 ? dispatchBallot<float>(a, s) : dispatchBallot<double>(a, s);
+}
+
+}  // namespace mkf

@@ -1,4 +1,5 @@
-// fused.cuh - arguments shared by the fused counting kernels (fused.cu, thermo.cu).
+// fused.cuh - arguments shared by the counting kernels (words.cuh, thermo.cu, thermo_tma.cu) and
+// their routing (fused.cu).
 #pragma once
 #include <vector>
 #include "mkf_common.cuh"
@@ -14,10 +15,9 @@ struct FusedArgs
    int D;                // planes of cells per slab
    int nSegX, nTileY, nSlabZ;
    long long nItems;     // nSegX * nTileY * nSlabZ warp work items
-   uint32_t gtm, eqm, ltm, nanP;  // GEN: per-threshold relation bits, map word of a NaN element
-   uint32_t nanRank;     // THERMO: rank of a NaN element
-   int rankHi;           // THERMO: rank counts thresholds <= f (else < f)
-   int complement;       // THERMO: stored codes are the bitwise complement of the true codes
+   uint32_t nanRank;     // rank of a NaN element
+   int rankHi;           // the rank counts thresholds <= f (else < f)
+   int complement;       // stored codes are the bitwise complement of the true codes
    uint64_t *out;        // [.][256] distributions
    int outRow[MKF_MAX_THRESH];  // output row of sorted threshold k
    double tlo[64];       // sorted thresholds for the "f > t" test, +inf padded
@@ -46,12 +46,12 @@ struct FieldTask
    double tlo[64], thi[64];
 };
 
-// Most thresholds the word-parallel kernels take in one read (more than two only when they share
-// one relation < <= > >=).
+// Most thresholds the word-parallel kernels take in one read (any relations).
 #ifndef WORDS_MAX_K
-#define WORDS_MAX_K 6
+#define WORDS_MAX_K 8
 #endif
 constexpr int kWordMaxK = WORDS_MAX_K;
+constexpr int kWordMaxDepth = 64;  // planes of cells per work item (untuned)
 
 // One field for the word-parallel kernels.
 struct WordTask
@@ -60,16 +60,15 @@ struct WordTask
    int64_t sx, sy, sz;    // element strides
    int X, Y, Z;
    int K;                 // 1 .. kWordMaxK
-   int cls[kWordMaxK];    // relation class per threshold (words.cu)
-   uint32_t m[kWordMaxK]; // relation masks
-   double tlo[kWordMaxK], thi[kWordMaxK];  // exact-equivalent thresholds for "f > t" / "f >= t" tests
+   int mode[kWordMaxK];   // tests of the map: bit 0 "f > tlo", bit 1 "f < thi"
    int outRow[kWordMaxK];
-   int complement;        // the map is counted negated: code c is stored in bin 255 - c
-   int variant;           // batched kernel: which instantiation counts this field
+   double tlo[kWordMaxK], thi[kWordMaxK];  // exact-equivalent thresholds of the two tests
+   uint32_t inv;          // bit k: threshold k is counted negated, code c is stored in bin 255 - c
+   int vec;               // rows and planes on 16-byte boundaries, unit x stride
    uint64_t *out;
    double *mom;           // moments kernel: [K][2 map values][sum f, sum f^2]
-   int D, pad_;           // planes of cells per work item
-   int nChunkX, nTileY, nSlabZ;
+   int D, W;              // planes of cells and tiles in x (words.cuh) per work item
+   int nStripX, nTileY, nSlabZ, pad_;
    long long nItems;
 };
 
@@ -79,6 +78,27 @@ struct BatchChunk
    int field, pad_;
    long long begin, end;
 };
+
+// Cut a batch's fields (tasks of one kernel) into chunks. A CTA waits for its slowest warp at the end
+// of a chunk and fills its copy pipeline anew at the start, so chunks are as long as leaves every
+// one of `ctas` CTAs about four, in multiples of its warps: with chunks of 64 items, 64 served fields
+// gave 29 and 65 chunks to 148 SMs (733 and 638 us).
+template <typename TASK>
+std::vector<BatchChunk> cutChunks(const std::vector<TASK> &tasks, int ctas, int warps, int maxItems)
+{
+   long long total = 0;
+   for (const TASK &t : tasks) { total += t.nItems; }
+   long long n = total / (4LL * ctas);
+   n = (n + warps - 1) / warps * warps;
+   n = n < warps ? warps : (n > maxItems ? maxItems : n);
+   std::vector<BatchChunk> chunks;
+   for (size_t f = 0; f < tasks.size(); f++) {
+      for (long long b = 0; b < tasks[f].nItems; b += n) {
+         chunks.push_back({(int)f, 0, b, b + n < tasks[f].nItems ? b + n : tasks[f].nItems});
+      }
+   }
+   return chunks;
+}
 
 struct BatchArgs
 {
@@ -97,13 +117,27 @@ struct WordBatchArgs
 };
 
 struct ConstEntry { int row, bin; };
-// Count one field for any thresholds (fused.cu): constant maps, one pass per relation class.
-// rowBase[i] is the output row of threshold i (NULL = identity).
-int fieldBPFD(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, int flags, cudaStream_t s, const int *rowBase);
+
+// A threshold set split into constant maps and varying thresholds (indices into the set, sorted by
+// value). cls: the relation all varying ones share (0 >, 1 >=, 2 <, 3 <=), negative when they differ
+// or it is = or !=.
+struct ThreshSplit
+{
+   int n, nConst, cls;
+   int idx[MKF_MAX_THRESH], constIdx[MKF_MAX_THRESH], constBin[MKF_MAX_THRESH];
+};
+void splitThresholds(const MKFThreshSet *pT, ThreshSplit &q);
+// Count the varying thresholds of a split, adding to out (no allocation, no clearing).
+int countVarying(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, cudaStream_t s);
+// Add `cells` to bin `bin` of output row `row`.
+int launchConstBin(uint64_t *out, int row, int bin, unsigned long long cells, cudaStream_t s);
+void floatBoundsPlain(double t, double &tlo, double &thi);
+// Count one field for any thresholds (fused.cu).
+int fieldBPFD(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, int flags, cudaStream_t s);
 
 enum { kPlanSingle = 0, kPlanThermo = 1, kPlanWords = 2 };
 // depth: planes of cells per work item; 0 = each kernel's default, -1 = chosen by field size.
-int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int rowBase, FieldTask &t, WordTask &w,
+int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, FieldTask &t, WordTask &w,
                    std::vector<ConstEntry> &consts, bool &anyVarying, int depth = 0);
 
 // Slab depth (planes of cells per work item) of a single-field launch of kernel family `family`
@@ -136,19 +170,30 @@ std::vector<ThermoGroup> groupThermoChunks(std::vector<BatchChunk> &chunks, cons
 int launchThermoGroups(const FieldTask *dTasks, const BatchChunk *dChunks, const std::vector<ThermoGroup> &groups,
                        unsigned *counters, int enc, cudaStream_t s);
 
-// Fill a word task's relation classes, batched variant and item grid (words.cu); launch the
-// batched word kernel over the chunks of tasks of one element type.
-void prepareWordTask(WordTask &a, int enc, int depth = 0);
-int launchWordsBatch(const WordBatchArgs &b, int enc, cudaStream_t s);
+// Fill a word task's field and its thresholds k0 .. k0 + n of a split (rows from row0).
+void fillWordTask(WordTask &w, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, int k0, int n, int row0);
+// Word tasks (words.cu): threshold t with relation mask m as the k-th of a task (inv zeroed
+// beforehand) whose counts go to output row `row`; the item grid for a slab depth and strip width.
+void fillWordThresh(WordTask &a, int k, int enc, double t, uint32_t m, int row);
+void fillWordGrid(WordTask &a, int enc, int depth, int strip);
 
-// Word-parallel kernel for one or two thresholds of any relations, or up to kWordMaxK thresholds of
-// one relation (words.cu); `masks` are the relation masks of f's (sorted) thresholds.
-// MKF_ERR_UNSUPPORTED otherwise.
-int launchWords(const FusedArgs &f, int enc, const uint32_t *masks, cudaStream_t s);
+// Count one field for a task's thresholds, 1 .. kWordMaxK of any relations (words.cu; fills the
+// task's item grid).
+int launchWords(WordTask &a, int enc, cudaStream_t s);
+
+// The same by warp votes, for one threshold; whether it is the faster one (ballot.cu).
+int launchBallots(WordTask &a, int enc, cudaStream_t s);
+bool useBallots(const WordTask &a, int enc);
 
 // Counts and descriptive moments of one or two thresholds (any relations) in one read (words.cu):
-// mom is device double[K][2][2], per threshold and map value the sum of f and of f^2.
-int launchWordsMoments(const FusedArgs &f, int enc, const uint32_t *masks, double *mom, cudaStream_t s);
+// a.mom is device double[K][2][2], per threshold and map value the sum of f and of f^2.
+int launchWordsMoments(WordTask &a, int enc, cudaStream_t s);
+
+// Chunks of the batched kernels' tasks (words_batch.cu, thermo.cu).
+std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks);
+std::vector<BatchChunk> thermoChunks(const std::vector<FieldTask> &tasks);
+// The batched word kernel over the chunks of tasks of one element type (words_batch.cu).
+int launchWordsBatch(const WordBatchArgs &b, int enc, cudaStream_t s);
 
 // Whether a pass's field and threshold count suit the TMA-staged rank-table kernel (thermo_tma.cu):
 // 3..16 thresholds, unit x stride, rows and planes on 16-byte boundaries, X >= 32, Y >= 9.

@@ -17,7 +17,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
-#include "mkf_common.cuh"
+#include "fused.cuh"
 
 #define MKF_NOALLOC_STAGE_BYTES ((size_t)32 << 20)
 #define MKF_NOALLOC_MAX_DEVICES 64
@@ -91,63 +91,9 @@ MKF_API int mkfFieldBPFDHostNoAlloc(uint64_t *pBPFDH, const MKFFieldDesc *pF, co
    cudaError_t e = cudaMemsetAsync(sc.counts, 0, (size_t)K * 256 * sizeof(uint64_t), s);
    if (e != cudaSuccess) { return cudaFail(e, "cudaMemsetAsync"); }
 
-   // classify the thresholds as the heap-using path does: constant maps, one thermometer class
-   // (every relation the same, one of > >= < <=) or the general per-threshold path
-   int constRow[MKF_MAX_THRESH], constBin[MKF_MAX_THRESH], nConst = 0;
-   int idx[MKF_MAX_THRESH], n = 0, cls0 = -2;
-   for (int i = 0; i < K; i++) {
-      const double t = pT->t[i];
-      const uint32_t m = (pT->m ? pT->m[i] : pT->mAll) & BMC_AL;
-      if (m == 0 || m == BMC_AL || std::isnan(t)) {
-         const bool one = (m == BMC_AL) || (std::isnan(t) && (m & BMC_EQ));
-         constRow[nConst] = i;
-         constBin[nConst++] = one ? 255 : 0;
-         continue;
-      }
-      int cls = -1;
-      if (m == BMC_GT) { cls = 0; }
-      else if (m == (BMC_GT | BMC_EQ)) { cls = 1; }
-      else if (m == BMC_LT) { cls = 2; }
-      else if (m == (BMC_LT | BMC_EQ)) { cls = 3; }
-      if (n == 0) { cls0 = cls; }
-      else if (cls != cls0) { cls0 = -1; }
-      idx[n++] = i;
-   }
-   // stable insertion sort of the thresholds by value
-   for (int a = 1; a < n; a++) {
-      const int v = idx[a];
-      int b = a - 1;
-      while (b >= 0 && pT->t[idx[b]] > pT->t[v]) { idx[b + 1] = idx[b]; b--; }
-      idx[b + 1] = v;
-   }
-   FusedPlain q;
-   memset(&q, 0, sizeof(q));
-   q.enc = pF->enc;
-   q.sx = 1;
-   q.sy = X;
-   q.sz = (int64_t)X * Y;
-   q.X = X;
-   q.Y = Y;
-   q.K = n;
-   q.out = (uint64_t *)sc.counts;
-   for (int k = 0; k < n; k++) {
-      const double t = pT->t[idx[k]];
-      if (pF->enc == ENC_F32) { floatBoundsPlain(t, q.tlo[k], q.thi[k]); }
-      else { q.tlo[k] = q.thi[k] = t; }
-      q.outRow[k] = idx[k];
-      const uint32_t m = (pT->m ? pT->m[idx[k]] : pT->mAll) & BMC_AL;
-      q.mask[k] = m;
-      q.gtm |= ((m >> 2) & 1u) << k;
-      q.eqm |= ((m >> 1) & 1u) << k;
-      q.ltm |= (m & 1u) << k;
-   }
-   q.thermo = (n > 0 && cls0 >= 0);
-   if (q.thermo) {
-      q.rankHi = (cls0 == 1 || cls0 == 2);
-      q.complement = (cls0 >= 2);
-      const bool eqBit = (cls0 == 1 || cls0 == 3);
-      q.nanRank = (eqBit != (q.complement != 0)) ? (uint32_t)n : 0u;
-   }
+   ThreshSplit q;
+   splitThresholds(pT, q);
+   MKFFieldDesc sub = *pF;
 
    if (cells > 0) {
       // slabs of S plane pairs (S+1 planes staged; the last plane is the next slab's first); no
@@ -155,17 +101,17 @@ MKF_API int mkfFieldBPFDHostNoAlloc(uint64_t *pBPFDH, const MKFFieldDesc *pF, co
       size_t S = MKF_NOALLOC_STAGE_BYTES / planeBytes - 1;
       if (S > (size_t)Z - 1) { S = (size_t)Z - 1; }
       const char *src = (const char *)pF->p;
-      for (size_t z0 = 0; n > 0 && z0 + 1 < (size_t)Z && rc == MKF_OK; z0 += S) {
+      for (size_t z0 = 0; q.n > 0 && z0 + 1 < (size_t)Z && rc == MKF_OK; z0 += S) {
          const size_t nPl = std::min(S + 1, (size_t)Z - z0);
          // same stream: this copy starts only after the previous slab's kernel has finished
          e = cudaMemcpyAsync(sc.stage, src + z0 * planeBytes, nPl * planeBytes, cudaMemcpyHostToDevice, s);
          if (e != cudaSuccess) { rc = cudaFail(e, "slab copy"); break; }
-         q.f = sc.stage;
-         q.Z = (int)nPl;
-         rc = launchFusedPlain(q, s);
+         sub.p = sc.stage;
+         sub.def[2] = (int32_t)nPl;
+         rc = countVarying((uint64_t *)sc.counts, &sub, pT, q, s);
       }
-      for (int c = 0; c < nConst && rc == MKF_OK; c++) {
-         rc = launchConstBin((uint64_t *)sc.counts, constRow[c], constBin[c], cells, s);
+      for (int c = 0; c < q.nConst && rc == MKF_OK; c++) {
+         rc = launchConstBin((uint64_t *)sc.counts, q.constIdx[c], q.constBin[c], cells, s);
       }
    }
    if (rc == MKF_OK) {

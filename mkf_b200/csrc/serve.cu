@@ -168,7 +168,6 @@ static int issueLaunch(MKFServer *s, LaunchSlot &sl)
    std::vector<Const> consts;
    struct Single { Request *r; MKFFieldDesc d; };
    std::vector<Single> singles;
-   constexpr int kChunk = 64;
    for (Request *r : sl.reqs) {
       MKFFieldDesc d = r->field;
       if (r->staged) {
@@ -196,20 +195,18 @@ static int issueLaunch(MKFServer *s, LaunchSlot &sl)
       for (const ConstEntry &c : ce) { consts.push_back({r->dCounts, c.row, c.bin, cells}); }
       if (kind == kPlanWords) {
          const int k = d.enc == ENC_F32 ? 0 : 1;
-         const int f = (int)wtasks[k].size();
-         for (long long b = 0; b < w.nItems; b += kChunk) { wchunks[k].push_back({f, 0, b, std::min<long long>(b + kChunk, w.nItems)}); }
          w.out = r->dCounts;
          wtasks[k].push_back(w);
       } else if (kind == kPlanThermo) {
          const int k = d.enc == ENC_F32 ? 0 : 1;
-         const int f = (int)tasks[k].size();
-         for (long long b = 0; b < t.nItems; b += kChunk) { chunks[k].push_back({f, 0, b, std::min<long long>(b + kChunk, t.nItems)}); }
          t.out = r->dCounts;
          tasks[k].push_back(t);
       }
    }
    std::vector<ThermoGroup> groups[2];  // thermometer chunks sorted into one run per kernel variant
    for (int k = 0; k < 2; k++) {
+      wchunks[k] = wordChunks(wtasks[k]);
+      chunks[k] = thermoChunks(tasks[k]);
       if (!chunks[k].empty()) { groups[k] = groupThermoChunks(chunks[k], tasks[k]); }
    }
    // one upload of the whole work list, segments 256-byte aligned:
@@ -267,7 +264,7 @@ static int issueLaunch(MKFServer *s, LaunchSlot &sl)
       ts.mAll = r->mAll;
       ts.t = r->t.data();
       ts.m = r->m.empty() ? nullptr : r->m.data();
-      rc = fieldBPFD(r->dCounts, &singles[i].d, &ts, MKF_F_ACCUMULATE, st, nullptr);
+      rc = fieldBPFD(r->dCounts, &singles[i].d, &ts, MKF_F_ACCUMULATE, st);
    }
    if (rc != MKF_OK) { return rc; }
    // counts wanted on the host: one pinned buffer per launch, copied out at completion

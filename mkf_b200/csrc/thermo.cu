@@ -373,6 +373,8 @@ bool prepareThermoTask(FieldTask &t, int enc, int depth)
    return true;
 }
 
+std::vector<BatchChunk> thermoChunks(const std::vector<FieldTask> &tasks) { return cutChunks(tasks, 3 * smCount(), kThWarps, 8 * kThWarps); }
+
 std::vector<ThermoGroup> groupThermoChunks(std::vector<BatchChunk> &chunks, const std::vector<FieldTask> &tasks)
 {
    std::vector<ThermoGroup> groups;

@@ -86,8 +86,6 @@ bool batchTuning()
    return gBatchTuning;
 }
 
-int fieldBPFD(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, int flags, cudaStream_t s, const int *rowBase);
-
 // One counting run of the field into a scratch buffer with depth / variant forced (0 / -1: not),
 // recording the kinds of launch it made; optionally timed (best of `reps`, ms).
 static int runOnce(const MKFFieldDesc *pF, const MKFThreshSet *pT, uint64_t *tmp, cudaStream_t s, int depth, int variant,
@@ -97,11 +95,11 @@ static int runOnce(const MKFFieldDesc *pF, const MKFThreshSet *pT, uint64_t *tmp
    tForceVariant = variant;
    tSeen = seen;
    if (seen) { seen->clear(); }
-   int rc = fieldBPFD(tmp, pF, pT, 0, s, nullptr);  // warm-up (and the launch kinds)
+   int rc = fieldBPFD(tmp, pF, pT, 0, s);  // warm-up (and the launch kinds)
    tSeen = nullptr;
    for (int rep = 0; rep < reps && rc == MKF_OK; rep++) {
       cudaError_t e = cudaEventRecord(e0, s);
-      if (e == cudaSuccess) { rc = fieldBPFD(tmp, pF, pT, 0, s, nullptr); }
+      if (e == cudaSuccess) { rc = fieldBPFD(tmp, pF, pT, 0, s); }
       if (rc == MKF_OK && e == cudaSuccess) { e = cudaEventRecord(e1, s); }
       if (rc == MKF_OK && e == cudaSuccess) { e = cudaEventSynchronize(e1); }
       float t = 0.0f;
