@@ -121,13 +121,15 @@ void fillWordTask(WordTask &w, const MKFFieldDesc *pF, const MKFThreshSet *pT, c
    }
 }
 
-// Split one field of a batch (rows from row0): one or two varying thresholds fill `w` for the
-// batched word kernel (returns kPlanWords); more thresholds that share one thermometer relation and
-// fit the rank table fill `t` for the batched thermometer kernel (kPlanThermo), unless the field has
-// kSoloVoxels or more: such a field fills the GPU on its own, and the single-field kernels (the
-// word kernel for a few thresholds, the TMA-staged rank table on aligned rows) count it faster than
-// the batched rank-table kernel. Those fields, and the rest, take the single-field path
-// (kPlanSingle). Constant maps are added to `consts`.
+// Split one field of a batch (rows from row0): one or two varying thresholds, or up to kWordMaxK of
+// any relations, fill `w` for the batched word kernel (returns kPlanWords); more thresholds that share
+// one thermometer relation and fit the rank table fill `t` for the batched thermometer kernel
+// (kPlanThermo). Fields of kSoloVoxels or more with more than two thresholds fill the GPU on their
+// own, and the single-field kernels (specialised on the number of thresholds; the TMA-staged rank table
+// on aligned rows) count them faster: those fields, and the rest, take the single-field path
+// (kPlanSingle). A served burst of 64 fields of 32^3 to 320^3 with 1-8 thresholds: word kernel up to 2
+// thresholds 1902 us, up to 8 1750; the cut at 2^24 voxels instead of 2^23 1800, at 2^26 2015. Constant
+// maps are added to `consts`.
 static constexpr double kSoloVoxels = (double)(1 << 23);
 int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, FieldTask &t, WordTask &w,
                    std::vector<ConstEntry> &consts, bool &anyVarying, int depth)
@@ -145,9 +147,9 @@ int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, Fie
    for (int c = 0; c < q.nConst; c++) { consts.push_back({row0 + q.constIdx[c], q.constBin[c]}); }
    anyVarying = q.n > 0;
    if (q.n == 0) { return kPlanSingle; }
-   if (q.n <= 2) {
+   if (q.n <= 2 || (q.n <= kWordMaxK && vox < kSoloVoxels)) {
       fillWordTask(w, pF, pT, q, 0, q.n, row0);
-      fillWordGrid(w, pF->enc, depth > 0 ? depth : 32, 2);
+      fillWordGrid(w, pF->enc, depth > 0 ? depth : 32, q.n <= 4 ? 2 : 1);
       return kPlanWords;
    }
    if (q.cls < 0 || vox >= kSoloVoxels) { return kPlanSingle; }

@@ -1,6 +1,8 @@
 // fused.cuh - arguments shared by the counting kernels (words.cuh, thermo.cu, thermo_tma.cu) and
 // their routing (fused.cu).
 #pragma once
+#include <algorithm>
+#include <utility>
 #include <vector>
 #include "mkf_common.cuh"
 
@@ -80,22 +82,24 @@ struct BatchChunk
 };
 
 // Cut a batch's fields (tasks of one kernel) into chunks. A CTA waits for its slowest warp at the end
-// of a chunk and fills its copy pipeline anew at the start, so chunks are as long as leaves every
-// one of `ctas` CTAs about four, in multiples of its warps: with chunks of 64 items, 64 served fields
-// gave 29 and 65 chunks to 148 SMs (733 and 638 us).
-template <typename TASK>
-std::vector<BatchChunk> cutChunks(const std::vector<TASK> &tasks, int ctas, int warps, int maxItems)
+// of a chunk and fills its copy pipeline anew at the start, so chunks are as long as leaves every one
+// of `ctas` CTAs about four of them, in multiples of its warps, and the costliest come first: with
+// chunks of 64 items, 64 served fields gave 29 and 65 chunks to 148 SMs (733 and 638 us). cost: of an
+// item of a task.
+template <typename TASK, typename COST>
+std::vector<BatchChunk> cutChunks(const std::vector<TASK> &tasks, int ctas, int warps, int maxItems, COST cost)
 {
-   long long total = 0;
-   for (const TASK &t : tasks) { total += t.nItems; }
-   long long n = total / (4LL * ctas);
-   n = (n + warps - 1) / warps * warps;
-   n = n < warps ? warps : (n > maxItems ? maxItems : n);
+   double total = 0.0;
+   for (const TASK &t : tasks) { total += (double)t.nItems * cost(t); }
+   std::vector<std::pair<double, int>> order;
+   for (size_t f = 0; f < tasks.size(); f++) { order.push_back({-cost(tasks[f]), (int)f}); }
+   std::stable_sort(order.begin(), order.end());
    std::vector<BatchChunk> chunks;
-   for (size_t f = 0; f < tasks.size(); f++) {
-      for (long long b = 0; b < tasks[f].nItems; b += n) {
-         chunks.push_back({(int)f, 0, b, b + n < tasks[f].nItems ? b + n : tasks[f].nItems});
-      }
+   for (const auto &o : order) {
+      const TASK &t = tasks[o.second];
+      long long n = (long long)(total / (4.0 * ctas) / -o.first / warps + 0.5) * warps;
+      n = n < warps ? warps : (n > maxItems ? maxItems : n);
+      for (long long b = 0; b < t.nItems; b += n) { chunks.push_back({o.second, 0, b, b + n < t.nItems ? b + n : t.nItems}); }
    }
    return chunks;
 }

@@ -373,7 +373,10 @@ bool prepareThermoTask(FieldTask &t, int enc, int depth)
    return true;
 }
 
-std::vector<BatchChunk> thermoChunks(const std::vector<FieldTask> &tasks) { return cutChunks(tasks, 3 * smCount(), kThWarps, 8 * kThWarps); }
+std::vector<BatchChunk> thermoChunks(const std::vector<FieldTask> &tasks) 
+{
+   return cutChunks(tasks, 3 * smCount(), kThWarps, 8 * kThWarps, [](const FieldTask &t) { return t.D + 1.0; });
+}
 
 std::vector<ThermoGroup> groupThermoChunks(std::vector<BatchChunk> &chunks, const std::vector<FieldTask> &tasks)
 {

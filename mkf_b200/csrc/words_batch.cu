@@ -52,7 +52,11 @@ __global__ void __launch_bounds__(kWdWarps * 32, 1) wordBatch(const __grid_const
    if (cur >= 0) { rowFlush(F, S); }
 }
 
-std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks) { return cutChunks(tasks, smCount(), kWdWarps, 16 * kWdWarps); }
+std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks) 
+{
+   // tiles of an item, each about half a threshold's work before the thresholds'
+   return cutChunks(tasks, smCount(), kWdWarps, 16 * kWdWarps, [](const WordTask &t) { return (t.D + 1.0) * t.W * (t.K + 0.5); });
+}
 
 template <typename T>
 static int launchBatchT(const WordBatchArgs &b, cudaStream_t s)

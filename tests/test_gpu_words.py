@@ -31,9 +31,9 @@ def test_word_kernel_tile_edges(mkf, oracle, cuda, dtype, shape):
             assert (got == want).all(), (k, off)
             if k <= 2:
                 assert (mkf.field_bpfd_moments(view, t, rel)[0].cpu().numpy().view(np.uint64) == want).all()
-                plan = mkf.BatchPlan([view, view], [t, t], [rel, rel])
-                assert (plan.launch().cpu().numpy().view(np.uint64) == np.concatenate([want, want])).all()
-                plan.close()
+            plan = mkf.BatchPlan([view, view], [t, t], [rel, rel])
+            assert (plan.launch().cpu().numpy().view(np.uint64) == np.concatenate([want, want])).all()
+            plan.close()
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
