@@ -1,5 +1,5 @@
-// ballot.cu - fused counting kernel for one threshold on fields of middle size: map words packed by
-// warp votes from registers.
+// ballot.cu - fused counting kernel for one threshold on fields of middle size, and for a few of
+// one test on larger FP64 fields: map words packed by warp votes from registers.
 //
 // The other kernel for few thresholds (words.cuh) lets each lane pack its own row from a copy of the
 // tile in shared memory. That costs fewer instructions per threshold, but a FP64 tile row holds only
@@ -7,7 +7,7 @@
 // A warp item is a tile of 32 x positions (31 cells), 32 rows (31 row pairs) and D planes, walked plane
 // by plane:
 //  * load: lane = x; the warp issues the 32 rows' coalesced loads at once;
-//  * pack: one ballot per row gives that row's 32-bit map word; lane r keeps row r's;
+//  * pack: one ballot per row and threshold gives that row's 32-bit map word; lane r keeps row r's;
 //  * count: lane = row pair. A cell's eight corners are bits b and b+1 of four words (this lane's
 //    row and the next lane's row, previous and current plane), so all-ones and all-zeros cells
 //    are popcounts of ANDs and ORs of the words and their one-bit shifts; only mixed cells form
@@ -38,10 +38,11 @@ __device__ __forceinline__ bool ballotBit(T v, T tlo, T thi)
 }
 
 // State of one warp item between planes: the previous plane's map words and the cell counts.
+template <int K>
 struct BallotCarry
 {
-   uint32_t pw = 0, pn = 0;  // previous plane: this lane's row word and the next row's
-   uint32_t n0 = 0, n1 = 0;  // all-zeros and all-ones cells counted by this lane
+   uint32_t pw[K], pn[K];  // previous plane: this lane's row word and the next row's
+   uint32_t n0[K], n1[K];  // all-zeros and all-ones cells counted by this lane
 };
 
 // Load one plane's 32 x 32 tile (lane = x). INNER: every row of the tile lies inside the field
@@ -62,43 +63,51 @@ __device__ __forceinline__ void loadPlane(T (&v)[32], const T *__restrict__ p, i
 }
 
 // Map, pack and count one plane (see the file comment). `first`: no previous plane yet.
-// `sRow` is the warp's 32-word transposition buffer.
-template <int MODE, typename T>
-__device__ __forceinline__ void countPlane(const T (&v)[32], BallotCarry &c, T tlo, T thi, bool xin, int lane, uint32_t vm, bool first,
-                                           uint32_t *sRow, uint32_t *sHist)
+// `sRow` is the warp's 32-word transposition buffer per threshold.
+template <int MODE, int K, typename T>
+__device__ __forceinline__ void countPlane(const T (&v)[32], BallotCarry<K> &c, const T (&tlo)[K], const T (&thi)[K], bool xin, int lane,
+                                           uint32_t vm, bool first, uint32_t (*sRow)[32], uint32_t *sHist)
 {
 #pragma unroll
    for (int r = 0; r < 32; r++) {
-      // every lane stores the same (warp-uniform) word
-      sRow[r] = __ballot_sync(FULL, xin && ballotBit<MODE>(v[r], tlo, thi));
-   }
-   __syncwarp();
-   const uint32_t cw = sRow[lane];
-   __syncwarp();
-   const uint32_t cn = __shfl_down_sync(FULL, cw, 1);
-   if (!first) {
-      const uint32_t a0 = c.pw, a1 = c.pn, a2 = cw, a3 = cn;
-      const uint32_t all = a0 & (a0 >> 1) & a1 & (a1 >> 1) & a2 & (a2 >> 1) & a3 & (a3 >> 1) & vm;
-      const uint32_t any = a0 | (a0 >> 1) | a1 | (a1 >> 1) | a2 | (a2 >> 1) | a3 | (a3 >> 1);
-      c.n1 += __popc(all);
-      c.n0 += __popc(vm & ~any);
-      uint32_t mixed = vm & any & ~all;
-      if (mixed) {
-         // word j's bits b, b+1 go to code bits 2j, 2j+1: pre-shift j's word left by 2j as a
-         // 64-bit (hi:lo) pair, so one funnel shift by b brings them into place
-         const uint32_t l1 = a1 << 2, h1 = a1 >> 30, l2 = a2 << 4, h2 = a2 >> 28, l3 = a3 << 6, h3 = a3 >> 26;
-         do {
-            const int b = 31 - __clz(mixed);
-            mixed ^= 1u << b;
-            uint32_t code = (__funnelshift_r(l1, h1, b) & ~3u) | ((a0 >> b) & 3u);
-            code = (__funnelshift_r(l2, h2, b) & ~15u) | (code & 15u);
-            code = (__funnelshift_r(l3, h3, b) & ~63u) | (code & 63u);
-            atomicAdd(sHist + (code & 255u), 1u);
-         } while (mixed);
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+         // every lane stores the same (warp-uniform) word
+         sRow[k][r] = __ballot_sync(FULL, xin && ballotBit<MODE>(v[r], tlo[k], thi[k]));
       }
    }
-   c.pw = cw;
-   c.pn = cn;
+   __syncwarp();
+   uint32_t cw[K];
+#pragma unroll
+   for (int k = 0; k < K; k++) { cw[k] = sRow[k][lane]; }
+   __syncwarp();
+#pragma unroll
+   for (int k = 0; k < K; k++) {
+      const uint32_t cn = __shfl_down_sync(FULL, cw[k], 1);
+      if (!first) {
+         const uint32_t a0 = c.pw[k], a1 = c.pn[k], a2 = cw[k], a3 = cn;
+         const uint32_t all = a0 & (a0 >> 1) & a1 & (a1 >> 1) & a2 & (a2 >> 1) & a3 & (a3 >> 1) & vm;
+         const uint32_t any = a0 | (a0 >> 1) | a1 | (a1 >> 1) | a2 | (a2 >> 1) | a3 | (a3 >> 1);
+         c.n1[k] += __popc(all);
+         c.n0[k] += __popc(vm & ~any);
+         uint32_t mixed = vm & any & ~all;
+         if (mixed) {
+            // word j's bits b, b+1 go to code bits 2j, 2j+1: pre-shift j's word left by 2j as a
+            // 64-bit (hi:lo) pair, so one funnel shift by b brings them into place
+            const uint32_t l1 = a1 << 2, h1 = a1 >> 30, l2 = a2 << 4, h2 = a2 >> 28, l3 = a3 << 6, h3 = a3 >> 26;
+            do {
+               const int b = 31 - __clz(mixed);
+               mixed ^= 1u << b;
+               uint32_t code = (__funnelshift_r(l1, h1, b) & ~3u) | ((a0 >> b) & 3u);
+               code = (__funnelshift_r(l2, h2, b) & ~15u) | (code & 15u);
+               code = (__funnelshift_r(l3, h3, b) & ~63u) | (code & 63u);
+               atomicAdd(sHist + k * 256 + (code & 255u), 1u);
+            } while (mixed);
+         }
+      }
+      c.pw[k] = cw[k];
+      c.pn[k] = cn;
+   }
 }
 
 // One warp counts work item `it` (31 x 31 cells, D planes) of field `a` into the CTA's histogram
@@ -107,9 +116,9 @@ __device__ __forceinline__ void countPlane(const T (&v)[32], BallotCarry &c, T t
 // already counted by the neighbouring tile are masked out), so no load needs clamping.
 // PF: the next plane's loads are issued before the current plane is counted (two plane buffers
 // in registers, alternating; INNER fields only).
-template <typename T, int MODE, bool INNER, bool PF>
-__device__ __forceinline__ void ballotItem(const WordTask &a, long long it, T tlo, T thi, uint32_t *sRow, uint32_t *sHist,
-                                           unsigned long long *sEnds)
+template <typename T, int MODE, int K, bool INNER, bool PF>
+__device__ __forceinline__ void ballotItem(const WordTask &a, long long it, const T (&tlo)[K], const T (&thi)[K], uint32_t (*sRow)[32],
+                                           uint32_t *sHist, unsigned long long (*sEnds)[2])
 {
    const int lane = threadIdx.x & 31;
    const T *__restrict__ F = (const T *)a.f;
@@ -132,62 +141,73 @@ __device__ __forceinline__ void ballotItem(const WordTask &a, long long it, T tl
    const uint32_t vm = (y0 + lane >= ys && y0 + lane < ye)
                           ? ((0xFFFFFFFFu >> (32 - (xe - x0))) & (0xFFFFFFFFu << (xs - x0)))
                           : 0u;
-   BallotCarry c;
+   BallotCarry<K> c;
+#pragma unroll
+   for (int k = 0; k < K; k++) { c.pw[k] = c.pn[k] = c.n0[k] = c.n1[k] = 0; }
    if (PF && INNER) {
       T va[32], vb[32];
       loadPlane<T, INNER>(va, base, a.sy, syb, nRow);
       for (int p = 0; p <= nPln; p += 2) {
          if (p + 1 <= nPln) { loadPlane<T, INNER>(vb, base + (long long)(p + 1) * a.sz, a.sy, syb, nRow); }
-         countPlane<MODE>(va, c, tlo, thi, xin, lane, vm, p == 0, sRow, sHist);
+         countPlane<MODE, K>(va, c, tlo, thi, xin, lane, vm, p == 0, sRow, sHist);
          if (p + 1 > nPln) { break; }
          if (p + 2 <= nPln) { loadPlane<T, INNER>(va, base + (long long)(p + 2) * a.sz, a.sy, syb, nRow); }
-         countPlane<MODE>(vb, c, tlo, thi, xin, lane, vm, false, sRow, sHist);
+         countPlane<MODE, K>(vb, c, tlo, thi, xin, lane, vm, false, sRow, sHist);
       }
    } else {
       for (int p = 0; p <= nPln; ++p) {
          T v[32];
          loadPlane<T, INNER>(v, base + (long long)p * a.sz, a.sy, syb, nRow);
-         countPlane<MODE>(v, c, tlo, thi, xin, lane, vm, p == 0, sRow, sHist);
+         countPlane<MODE, K>(v, c, tlo, thi, xin, lane, vm, p == 0, sRow, sHist);
       }
    }
-   const unsigned long long s0 = __reduce_add_sync(FULL, c.n0);
-   const unsigned long long s1 = __reduce_add_sync(FULL, c.n1);
-   if (lane == 0) {
-      if (s0) { atomicAdd(&sEnds[0], s0); }
-      if (s1) { atomicAdd(&sEnds[1], s1); }
+#pragma unroll
+   for (int k = 0; k < K; k++) {
+      const unsigned long long s0 = __reduce_add_sync(FULL, c.n0[k]);
+      const unsigned long long s1 = __reduce_add_sync(FULL, c.n1[k]);
+      if (lane == 0) {
+         if (s0) { atomicAdd(&sEnds[k][0], s0); }
+         if (s1) { atomicAdd(&sEnds[k][1], s1); }
+      }
    }
 }
 
-template <typename T, int MODE, bool INNER, int MINB, bool PF>
+template <typename T, int MODE, int K, bool INNER, int MINB, bool PF>
 __global__ void __launch_bounds__(kBlWarps * 32, MINB) ballotBPFD(const __grid_constant__ WordTask a)
 {
-   __shared__ uint32_t sHist[256];
-   __shared__ unsigned long long sEnds[2];  // all-zeros, all-ones cells
-   __shared__ uint32_t sRows[kBlWarps][32];
-   for (int i = threadIdx.x; i < 256; i += blockDim.x) { sHist[i] = 0; }
-   if (threadIdx.x < 2) { sEnds[threadIdx.x] = 0; }
+   __shared__ uint32_t sHist[K * 256];
+   __shared__ unsigned long long sEnds[K][2];  // all-zeros, all-ones cells
+   __shared__ uint32_t sRows[kBlWarps][K][32];
+   for (int i = threadIdx.x; i < K * 256; i += blockDim.x) { sHist[i] = 0; }
+   if (threadIdx.x < K * 2) { (&sEnds[0][0])[threadIdx.x] = 0; }
    __syncthreads();
-   const T tlo = (T)a.tlo[0], thi = (T)a.thi[0];
+   T tlo[K], thi[K];
+#pragma unroll
+   for (int k = 0; k < K; k++) {
+      tlo[k] = (T)a.tlo[k];
+      thi[k] = (T)a.thi[k];
+   }
    const long long gw = (long long)blockIdx.x * kBlWarps + (threadIdx.x >> 5);
    const long long nw = (long long)gridDim.x * kBlWarps;
    for (long long it = gw; it < a.nItems; it += nw) {
-      ballotItem<T, MODE, INNER, PF>(a, it, tlo, thi, sRows[threadIdx.x >> 5], sHist, sEnds);
+      ballotItem<T, MODE, K, INNER, PF>(a, it, tlo, thi, sRows[threadIdx.x >> 5], sHist, sEnds);
    }
    __syncthreads();
    // mixed codes as counted, 0 / 255 from the totals; counted negated, code c belongs in bin 255 - c
-   for (int c = threadIdx.x; c < 256; c += blockDim.x) {
-      unsigned long long v = sHist[c];
-      if (c == 0) { v += sEnds[0]; }
-      if (c == 255) { v += sEnds[1]; }
-      if (v) { atomicAdd((unsigned long long *)(a.out + (size_t)a.outRow[0] * 256 + ((a.inv & 1u) ? 255 - c : c)), v); }
+   for (int i = threadIdx.x; i < K * 256; i += blockDim.x) {
+      const int k = i >> 8, c = i & 255;
+      unsigned long long v = sHist[i];
+      if (c == 0) { v += sEnds[k][0]; }
+      if (c == 255) { v += sEnds[k][1]; }
+      if (v) { atomicAdd((unsigned long long *)(a.out + (size_t)a.outRow[k] * 256 + ((a.inv >> k) & 1u ? 255 - c : c)), v); }
    }
 }
 
-template <typename T, int MODE, bool INNER, int MINB, bool PF>
+template <typename T, int MODE, int K, bool INNER, int MINB, bool PF>
 static int launchBallotT(const WordTask &a, cudaStream_t s)
 {
    static std::atomic<int> occ{0};
-   auto kern = ballotBPFD<T, MODE, INNER, MINB, PF>;
+   auto kern = ballotBPFD<T, MODE, K, INNER, MINB, PF>;
    const int blocksPerSM = cachedOccupancy(occ, kern, kBlWarps * 32, 0);
    long long grid = (a.nItems + kBlWarps - 1) / kBlWarps;
    const long long cap = (long long)smCount() * blocksPerSM;
@@ -197,35 +217,55 @@ static int launchBallotT(const WordTask &a, cudaStream_t s)
    return cudaFail(cudaGetLastError(), "ballotBPFD launch");
 }
 
-template <typename T, int MODE>
-static int launchBallotM(const WordTask &a, cudaStream_t s)
+static bool innerTiles(const WordTask &a, int enc)
 {
-   const int64_t syb = a.sy * (int64_t)sizeof(T);
-   const bool inner = a.X >= 32 && a.Y >= 32 && syb > 0 && syb * 31 < (int64_t)1 << 32;
+   const int64_t syb = a.sy * (enc == ENC_F32 ? 4 : 8);
+   return a.X >= 32 && a.Y >= 32 && syb > 0 && syb * 31 < (int64_t)1 << 32;
+}
+
+template <typename T, int MODE>
+static int launchBallotM(const WordTask &a, int enc, cudaStream_t s)
+{
    constexpr bool F32 = sizeof(T) == 4;
-   if (!inner) { return launchBallotT<T, MODE, false, 2, false>(a, s); }
-   if (F32 && a.D >= kBlPfDepth) { return launchBallotT<T, MODE, true, 2, F32>(a, s); }
-   return launchBallotT<T, MODE, true, F32 ? 4 : 2, false>(a, s);
+   if constexpr (!F32 && MODE < 3) {
+      if (a.K == 2) { return launchBallotT<T, MODE, 2, true, 2, false>(a, s); }
+      if (a.K == 3) { return launchBallotT<T, MODE, 3, true, 2, false>(a, s); }
+      if (a.K == 4) { return launchBallotT<T, MODE, 4, true, 2, false>(a, s); }
+      if (a.K == 5) { return launchBallotT<T, MODE, 5, true, 2, false>(a, s); }
+   }
+   if (!innerTiles(a, enc)) { return launchBallotT<T, MODE, 1, false, 2, false>(a, s); }
+   if (F32 && a.D >= kBlPfDepth) { return launchBallotT<T, MODE, 1, true, 2, F32>(a, s); }
+   return launchBallotT<T, MODE, 1, true, F32 ? 4 : 2, false>(a, s);
 }
 
 template <typename T>
-static int dispatchBallot(const WordTask &a, cudaStream_t s)
+static int dispatchBallot(const WordTask &a, int enc, cudaStream_t s)
 {
    switch (a.mode[0]) {
-      case 1: return launchBallotM<T, 1>(a, s);
-      case 2: return launchBallotM<T, 2>(a, s);
-      default: return launchBallotM<T, 3>(a, s);
+      case 1: return launchBallotM<T, 1>(a, enc, s);
+      case 2: return launchBallotM<T, 2>(a, enc, s);
+      default: return launchBallotM<T, 3>(a, enc, s);
    }
 }
 
 // B200, device time of a call, this kernel against the other (words.cuh): FP32 64^3 7.9 / 6.9 us,
 // 128^3 8.3 / 8.9, 256^3 18.8 / 20.2, 301 x 333 x 277 33.7 / 34.6, 512^3 115 / 109,
 // 128 x 2048 x 2048 398 / 359; FP64 64^3 8.0 / 6.1, 128^3 9.2 / 9.6, 256 x 512 x 512 86 / 97,
-// 333 x 401 x 487 85 / 111. With two thresholds the other is faster from 512^3 on and in small fields.
+// 333 x 401 x 487 85 / 111. Four thresholds on larger FP64 fields: 256 x 512 x 512 plane waves 131 / 146,
+// GRF 158 / 161. Two to five on FP64 rows off 16-byte boundaries, where the other kernel's tile rows are
+// a ninth wider and fewer warps fit: 333 x 401 x 487 GRF, 3 thresholds 155 / 170, 4 158 / 181, plane
+// waves, 5 (against the rank table) 163 / 190; 301 x 333 x 277, 2 61 / 64, 3 82 / 79, 4 85 / 87;
+// 100 x 101 x 99, 3 18 / 12.
 bool useBallots(const WordTask &a, int enc)
 {
    const double voxels = (double)a.X * a.Y * a.Z;
-   return a.K == 1 && voxels >= (double)(1 << 20) && (enc == ENC_F64 || voxels < (double)(1 << 26));
+   if (a.K == 1) { return voxels >= (double)(1 << 20) && (enc == ENC_F64 || voxels < (double)(1 << 26)); }
+   if (enc != ENC_F64 || a.K > 5 || voxels < (double)(1 << 24) || !innerTiles(a, enc)) { return false; }
+   if (a.K != 4 && wordRowsAligned(a, enc)) { return false; }
+   for (int k = 0; k < a.K; k++) {
+      if (a.mode[k] != a.mode[0] || a.mode[k] == 3) { return false; }
+   }
+   return true;
 }
 
 int launchBallots(WordTask &a, int enc, cudaStream_t s)
@@ -236,7 +276,7 @@ int launchBallots(WordTask &a, int enc, cudaStream_t s)
                     sizeDepth(kBlD, (long long)a.nStripX * a.nTileY, a.Z, (long long)smCount() * kBlItemsPerSM));
    a.nSlabZ = (a.Z - 1 + a.D - 1) / a.D;
    a.nItems = (long long)a.nStripX * a.nTileY * a.nSlabZ;
-   return enc == ENC_F32 ? dispatchBallot<float>(a, s) : dispatchBallot<double>(a, s);
+   return enc == ENC_F32 ? dispatchBallot<float>(a, enc, s) : dispatchBallot<double>(a, enc, s);
 }
 
 }  // namespace mkf

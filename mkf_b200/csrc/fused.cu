@@ -73,12 +73,18 @@ void splitThresholds(const MKFThreshSet *pT, ThreshSplit &q)
    }
 }
 
-// Thresholds of one relation that the word kernel counts rather than a rank-table kernel, whose cost
+// Thresholds of one relation that the word kernels count rather than a rank-table kernel, whose cost
 // hardly grows with their number (B200, us, word kernel / rank table): 512^3 FP32 GRF 4 thresholds
 // 244 / 302, 5 325 / 304; 128 x 2048 x 2048 FP32 plane waves 4 739 / 734, 5 947 / 1145; 256 x 512 x 512
-// FP64 GRF 4 162 / 158 (word kernel by votes), 5 221 / 166; 301 x 333 x 277 FP32 (rows off 16 bytes) 6
-// 96 / 107, 8 127 / 110; 333 x 401 x 487 FP64 6 296 / 226.
-static int wordThresholds(int enc, bool tmaRows) { return tmaRows ? 4 : (enc == ENC_F32 ? 6 : 4); }
+// FP64 GRF 4 158 / 165, 5 221 / 166; rows off 16-byte boundaries: 301 x 333 x 277 FP32 4 72 / 76, 5 83 / 76,
+// 6 95 / 76; 333 x 401 x 487 FP64 4 158 / 192, 5 192 / 193, plane waves 163 / 190;
+// 301 x 333 x 277 FP64 5 104 / 88.
+static int wordThresholds(const FusedArgs &a, int enc)
+{
+   const bool large = (double)a.X * a.Y * a.Z >= (double)(1 << 25);
+   return enc == ENC_F64 && large && !tmaRowsAligned(a, enc) ? 5 : 4;
+}
+
 
 void fillRankArgs(FusedArgs &a, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, int row0)
 {
@@ -170,11 +176,11 @@ int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, Fie
 
 int countVarying(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, cudaStream_t s)
 {
-   if (q.cls >= 0 && q.n > 2) {
+   if (q.cls >= 0 && q.n > 4) {
       FusedArgs a;
       fillRankArgs(a, pF, pT, q, 0);
       a.out = out;
-      if (q.n > wordThresholds(pF->enc, tmaRowsAligned(a, pF->enc))) {
+      if (q.n > wordThresholds(a, pF->enc)) {
          const int rc = launchThermo(a, pF->enc, s);
          if (rc != MKF_ERR_UNSUPPORTED) { return rc; }
       }

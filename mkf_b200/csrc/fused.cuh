@@ -179,13 +179,15 @@ void fillWordTask(WordTask &w, const MKFFieldDesc *pF, const MKFThreshSet *pT, c
 // Word tasks (words.cu): threshold t with relation mask m as the k-th of a task (inv zeroed
 // beforehand) whose counts go to output row `row`; the item grid for a slab depth and strip width.
 void fillWordThresh(WordTask &a, int k, int enc, double t, uint32_t m, int row);
+bool wordRowsAligned(const WordTask &a, int enc);  // unit x stride, rows and planes on 16-byte boundaries
 void fillWordGrid(WordTask &a, int enc, int depth, int strip);
 
 // Count one field for a task's thresholds, 1 .. kWordMaxK of any relations (words.cu; fills the
 // task's item grid).
 int launchWords(WordTask &a, int enc, cudaStream_t s);
 
-// The same by warp votes, for one threshold; whether it is the faster one (ballot.cu).
+// The same by warp votes, for one threshold or a few of one test; whether it is the faster one
+// (ballot.cu).
 int launchBallots(WordTask &a, int enc, cudaStream_t s);
 bool useBallots(const WordTask &a, int enc);
 

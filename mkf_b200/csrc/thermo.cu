@@ -465,16 +465,13 @@ int launchThermo(FusedArgs &a, int enc, cudaStream_t s)
    a.lutC = prepareKeys(a, enc);
    if (a.lutC == 0) { return MKF_ERR_UNSUPPORTED; }
    const long long perPlane = (long long)((a.X - 1 + 30) / 31) * ((a.Y - 1 + THERMO_TY - 1) / THERMO_TY);
-#ifndef MKF_NO_TMA
-   // the TMA-staged kernel where the field allows it (up to 16 thresholds, 16-byte aligned rows)
-   a.D = THERMO_D;
-   if (thermoTmaEligible(a, enc)) {
+   // up to 16 thresholds on fields of at least one tile: tiles staged in shared memory
+   if (thermoRingEligible(a)) {
       itemGrid(a, tunedDepth(kFamThermoTma, enc, a.K, a.X, a.Y, a.Z,
                              sizeDepth(THERMO_D, perPlane, a.Z, (long long)smCount() * kTmItemsPerSM)));
-      const int rc = launchThermoTma(a, enc, tunedVariant(kFamThermoTma, enc, a.K, a.X, a.Y, a.Z, 0), s);
+      const int rc = launchThermoRing(a, enc, tunedVariant(kFamThermoTma, enc, a.K, a.X, a.Y, a.Z, 0), s);
       if (rc != MKF_ERR_UNSUPPORTED) { return rc; }
    }
-#endif
    itemGrid(a, tunedDepth(kFamThermo, enc, a.K, a.X, a.Y, a.Z,
                           sizeDepth(THERMO_D, perPlane, a.Z, (long long)smCount() * kThItemsPerSM)));
    const bool ge = a.rankHi != 0, inner = innerTiles(a, enc);

@@ -323,12 +323,12 @@ __device__ __forceinline__ uint32_t cellCode(uint32_t R0, uint32_t R1, uint32_t 
    return gatherCode((((R0 + C) >> 4) & 0x08080808u) | ((R1 + C) & 0x80808080u));
 }
 
-// The TMA-staged rank-table kernel (thermo_tma.cu): whether it takes this pass (after prepareKeys
-// and itemGrid), and its launch (MKF_ERR_UNSUPPORTED when it does not take it).
+// The rank-table kernel with its tiles staged in shared memory (thermo_tma.cu): whether it takes this
+// pass (after prepareKeys), and its launch (after itemGrid; MKF_ERR_UNSUPPORTED when it does not).
 static constexpr int kTmItemsPerSM = 80;  // four items per resident warp (20 per SM)
-bool thermoTmaEligible(const FusedArgs &a, int enc);
+bool thermoRingEligible(const FusedArgs &a);
 // variant: CTA shape, histogram privatisation and queue kind (kTmVariants in thermo_tma.cu,
-// kTmNumVariants of them), 0 = default.
-int launchThermoTma(const FusedArgs &a, int enc, int variant, cudaStream_t s);
+// kTmNumVariants of them), 0 = default; fields off 16-byte boundaries have the default only.
+int launchThermoRing(const FusedArgs &a, int enc, int variant, cudaStream_t s);
 
 }  // namespace mkf

@@ -1,5 +1,6 @@
-// thermo_tma.cu - the rank-table counting kernel with plane tiles staged by TMA, for 3..16
-// thresholds of one relation (< <= > >=) on fields whose rows start on 16-byte boundaries.
+// thermo_tma.cu - the rank-table counting kernel with plane tiles staged in shared memory (by TMA on
+// fields whose rows start on 16-byte boundaries, else by cp.async), for 3..16 thresholds of one relation
+// (< <= > >=).
 //
 // The method is thermo.cu's (sorted thresholds: an element's K map bits are a thermometer, found
 // as a rank through a table over order-preserving keys; a cell is all-ones below its smallest
@@ -242,7 +243,12 @@ __device__ __forceinline__ TmItem itemOf(const FusedArgs &a, long long it, int l
    return m;
 }
 
-template <typename T, bool GE, int CMAX, int V>
+// TMA false: fields that a tensor map cannot take (rows off 16-byte boundaries, strided x). Every lane
+// then copies its own column of the tile with cp.async, one element per row, into the same ring, and
+// waits for its own copies only; the rest is the same. Against thermo.cu, which took these fields
+// before (B200, us): 333 x 401 x 487 FP64, 12 thresholds 240 -> 197, 16 265 -> 212; 301 x 333 x 277 FP32, 8
+// 110 -> 77; 100 x 101 x 99 FP64, 12 27 -> 18.
+template <typename T, bool GE, int CMAX, int V, bool TMA>
 __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
     thermoTmaBPFD(const __grid_constant__ FusedArgs a, const __grid_constant__ CUtensorMap tm)
 {
@@ -265,7 +271,7 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    unsigned char *ring = dsm + histBytes + ((128u - (histEnd & 127u)) & 127u);
    uint2 *queue = reinterpret_cast<uint2 *>(ring + (size_t)kTmWarps * S * G::PITCH) + warp * G::QWORDS;
 
-   if (lane == 0) {
+   if (TMA && lane == 0) {
       for (int s = 0; s < S; s++) { mbarInit((uint32_t)__cvta_generic_to_shared(&bars[warp][s]), 1); }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
    }
@@ -283,26 +289,41 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    // producer cursor (every lane tracks it; lane 0 issues): item, plane, tile coordinates
    long long pIt = first;
    int pP = 0, pX = 0, pY = 0, pZ = 0, pN = -1;
-   if (pIt < a.nItems) {
-      const TmItem m = itemOf<G::ALIGN>(a, pIt, lane);
-      pX = m.xa; pY = m.y0; pZ = m.z0; pN = m.nPln;
-   }
-   uint32_t gp = 0;  // planes issued by this warp
-   auto issue = [&]() {
-      if (pIt >= a.nItems) { return; }
-      if (lane == 0) {
-         const uint32_t st = gp % S;
-         tmaTile3D(&tm, ringW + st * G::PITCH, bar0 + 8u * st, pX, pY, pZ + pP, G::BYTES);
-      }
-      ++gp;
-      if (++pP > pN) {
-         pIt += nw;
-         pP = 0;
-         if (pIt < a.nItems) {
-            const TmItem m = itemOf<G::ALIGN>(a, pIt, lane);
-            pX = m.xa; pY = m.y0; pZ = m.z0; pN = m.nPln;
+   const char *pCol = nullptr;  // (not TMA) this lane's element of the tile's first row
+   auto begin = [&]() {
+      if (pIt < a.nItems) {
+         const TmItem m = itemOf<G::ALIGN>(a, pIt, lane);
+         pX = m.xa; pY = m.y0; pZ = m.z0; pN = m.nPln;
+         if (!TMA) {
+            pCol = (const char *)a.f + ((int64_t)(m.xa + m.xoff + lane) * a.sx + (int64_t)m.y0 * a.sy + (int64_t)m.z0 * a.sz) * (int64_t)sizeof(T);
          }
       }
+   };
+   begin();
+   uint32_t gp = 0;  // planes issued by this warp
+   auto issue = [&]() {
+      if (pIt < a.nItems) {
+         const uint32_t st = gp % S;
+         if (TMA) {
+            if (lane == 0) { tmaTile3D(&tm, ringW + st * G::PITCH, bar0 + 8u * st, pX, pY, pZ + pP, G::BYTES); }
+         } else {
+            const uint32_t dst = ringW + st * G::PITCH + (uint32_t)(lane * (int)sizeof(T));
+            const char *q = pCol;
+#pragma unroll
+            for (int j = 0; j < kTmRows; ++j) {
+               asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + (uint32_t)(j * G::BX * (int)sizeof(T))), "l"(q), "n"((int)sizeof(T)) : "memory");
+               q += a.sy * (int64_t)sizeof(T);
+            }
+            pCol += a.sz * (int64_t)sizeof(T);
+         }
+         ++gp;
+         if (++pP > pN) {
+            pIt += nw;
+            pP = 0;
+            begin();
+         }
+      }
+      if (!TMA) { asm volatile("cp.async.commit_group;" ::: "memory"); }
    };
    for (int s = 0; s + 1 < S; s++) { issue(); }
 
@@ -311,10 +332,14 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    // wait for plane g's tile, rank the lane's column (9 rows), refill the stage of plane g - 1
    auto plane = [&](int xoff, uint32_t (&r)[kTmRows]) -> bool {
       const uint32_t st = g % S;
-      // (the warp leaves together: every lane's wait must have seen the copy)
-      if (!__all_sync(FULL, mbarWait(bar0 + 8u * st, (g / S) & 1u))) { return false; }
+      if (TMA) {
+         // (the warp leaves together: every lane's wait must have seen the copy)
+         if (!__all_sync(FULL, mbarWait(bar0 + 8u * st, (g / S) & 1u))) { return false; }
+      } else {
+         asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+      }
       // this lane's column of the plane tile (the mbarrier wait orders these loads after the copy)
-      const T *col = reinterpret_cast<const T *>(ring + (size_t)(warp * S + (int)st) * G::PITCH) + xoff + lane;
+      const T *col = reinterpret_cast<const T *>(ring + (size_t)(warp * S + (int)st) * G::PITCH) + (TMA ? xoff : 0) + lane;
       const uint32_t *colW = reinterpret_cast<const uint32_t *>(col) + (W - 1);
       bool slow = false;   // a FP64 high word equal to a threshold's
       uint32_t rOr = 0;    // slow-path buckets rank above 32
@@ -553,12 +578,12 @@ unsigned thermoTmaFaults(bool clear)
    return v;
 }
 
-template <typename T, bool GE, int CMAX, int V>
+template <typename T, bool GE, int CMAX, int V, bool TMA>
 static int launchTmaT(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
 {
    using G = TmaGeom<T, V>;
    static std::atomic<int> occ[kTmMaxK + 1];
-   auto kern = thermoTmaBPFD<T, GE, CMAX, V>;
+   auto kern = thermoTmaBPFD<T, GE, CMAX, V, TMA>;
    const size_t smem = tmaDynBytes<T, V>(a.K);
    const int blocksPerSM = cachedOccupancy(occ[a.K], kern, G::WARPS * 32, smem, tmaDynBytes<T, V>(kTmMaxK));
    long long grid = (a.nItems + G::WARPS - 1) / G::WARPS;
@@ -569,16 +594,18 @@ static int launchTmaT(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
    return cudaFail(cudaGetLastError(), "thermoTmaBPFD launch");
 }
 
-// Thresholds sharing rank-table buckets (four candidates) take the default variant only.
+// Thresholds sharing rank-table buckets (four candidates), and fields without a tensor map, take the
+// default variant only.
 template <typename T, bool GE>
-static int launchTmaG(const FusedArgs &a, const CUtensorMap &tm, int variant, cudaStream_t s)
+static int launchTmaG(const FusedArgs &a, const CUtensorMap &tm, bool tma, int variant, cudaStream_t s)
 {
-   if (a.lutC > 1) { return launchTmaT<T, GE, 4, 0>(a, tm, s); }
+   if (!tma) { return a.lutC > 1 ? launchTmaT<T, GE, 4, 0, false>(a, tm, s) : launchTmaT<T, GE, 1, 0, false>(a, tm, s); }
+   if (a.lutC > 1) { return launchTmaT<T, GE, 4, 0, true>(a, tm, s); }
    switch (variant) {
-      case 1: return launchTmaT<T, GE, 1, 1>(a, tm, s);
-      case 2: return launchTmaT<T, GE, 1, 2>(a, tm, s);
-      case 3: return launchTmaT<T, GE, 1, 3>(a, tm, s);
-      default: return launchTmaT<T, GE, 1, 0>(a, tm, s);
+      case 1: return launchTmaT<T, GE, 1, 1, true>(a, tm, s);
+      case 2: return launchTmaT<T, GE, 1, 2, true>(a, tm, s);
+      case 3: return launchTmaT<T, GE, 1, 3, true>(a, tm, s);
+      default: return launchTmaT<T, GE, 1, 0, true>(a, tm, s);
    }
 }
 
@@ -589,23 +616,21 @@ bool tmaRowsAligned(const FusedArgs &a, int enc)
           (a.sy * esz) % 16 == 0 && (a.sz * esz) % 16 == 0 && a.sy >= a.X && a.sz >= a.sy * a.Y && encodeFn() != nullptr;
 }
 
-bool thermoTmaEligible(const FusedArgs &a, int enc)
+bool thermoRingEligible(const FusedArgs &a)
 {
-   return tmaRowsAligned(a, enc) && a.lutC >= 1 && a.D >= 1 && a.D <= kTmMaxDepth;
+   return a.K > 2 && a.K <= kTmMaxK && a.X >= 32 && a.Y >= 9 && a.Z >= 2 && a.lutC >= 1;
 }
 
 // a.tkey / a.lutC filled (prepareKeys) and the item grid set for 8-row items (itemGrid).
-int launchThermoTma(const FusedArgs &a, int enc, int variant, cudaStream_t s)
+int launchThermoRing(const FusedArgs &a, int enc, int variant, cudaStream_t s)
 {
-   if (!thermoTmaEligible(a, enc)) { return MKF_ERR_UNSUPPORTED; }
-   const bool f32 = enc == ENC_F32;
-   CUtensorMap tm;
-   if (!encodeField3D(&tm, a.f, enc, a.X, a.Y, a.Z, a.sy, a.sz, f32 ? TmaGeom<float>::BX : TmaGeom<double>::BX, kTmRows)) {
-      return MKF_ERR_UNSUPPORTED;
-   }
-   const bool ge = a.rankHi != 0;
-   if (f32) { return ge ? launchTmaG<float, true>(a, tm, variant, s) : launchTmaG<float, false>(a, tm, variant, s); }
-   return ge ? launchTmaG<double, true>(a, tm, variant, s) : launchTmaG<double, false>(a, tm, variant, s);
+   if (!thermoRingEligible(a) || a.D < 1 || a.D > kTmMaxDepth) { return MKF_ERR_UNSUPPORTED; }
+   const bool f32 = enc == ENC_F32, ge = a.rankHi != 0;
+   CUtensorMap tm = {};
+   const bool tma = tmaRowsAligned(a, enc) &&
+                    encodeField3D(&tm, a.f, enc, a.X, a.Y, a.Z, a.sy, a.sz, f32 ? TmaGeom<float>::BX : TmaGeom<double>::BX, kTmRows);
+   if (f32) { return ge ? launchTmaG<float, true>(a, tm, tma, variant, s) : launchTmaG<float, false>(a, tm, tma, variant, s); }
+   return ge ? launchTmaG<double, true>(a, tm, tma, variant, s) : launchTmaG<double, false>(a, tm, tma, variant, s);
 }
 
 }  // namespace mkf

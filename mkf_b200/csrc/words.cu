@@ -46,11 +46,16 @@ void fillWordThresh(WordTask &a, int k, int enc, double t, uint32_t m, int row)
    a.outRow[k] = row;
 }
 
-void fillWordGrid(WordTask &a, int enc, int depth, int strip)
+bool wordRowsAligned(const WordTask &a, int enc)
 {
    const int64_t b = enc == ENC_F32 ? 4 : 8;
+   return a.sx == 1 && ((uintptr_t)a.f % 16) == 0 && (a.sy * b) % 16 == 0 && (a.sz * b) % 16 == 0;
+}
+
+void fillWordGrid(WordTask &a, int enc, int depth, int strip)
+{
    const int el = enc == ENC_F32 ? 32 : 16;
-   a.vec = a.sx == 1 && ((uintptr_t)a.f % 16) == 0 && (a.sy * b) % 16 == 0 && (a.sz * b) % 16 == 0;
+   a.vec = wordRowsAligned(a, enc);
    const int tiles = (a.X - 1 + el - 1) / el;
    a.W = strip;
    a.nStripX = (tiles + strip - 1) / strip;
