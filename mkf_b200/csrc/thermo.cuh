@@ -216,8 +216,9 @@ __host__ __device__ constexpr size_t thermoDynBytes(int K)
 
 // Load one field's thresholds, build its rank table and clear the histogram (whole CTA).
 // copyRows: histogram rows per copy (K, or more when rows past K take discarded counts);
-// copies: histogram copies.
-template <typename P>
+// copies: histogram copies. RAW: the table is indexed by the ranked word's own top bits instead of its
+// order-preserving key's.
+template <bool RAW = false, typename P>
 __device__ void ctaSetup(const P &a, ThermoShared &S, uint32_t *hist, int copyRows = 0, int copies = kHistCopies)
 {
    const int K = a.K;
@@ -236,13 +237,15 @@ __device__ void ctaSetup(const P &a, ThermoShared &S, uint32_t *hist, int copyRo
       uint32_t word = 0;
 #pragma unroll
       for (int q = 0; q < 4; q++) {
-         const uint32_t start = (uint32_t)(4 * w + q) << kLutShift;
+         const uint32_t bits = 4 * w + q;
+         const uint32_t b = RAW ? bits ^ (bits & (kLutSize / 2) ? kLutSize - 1 : kLutSize / 2) : bits;
+         const uint32_t start = b << kLutShift;
          int lo = 0, hi = K;  // first key >= start
          while (lo < hi) {
             const int mid = (lo + hi) >> 1;
             if (S.key[mid] < start) { lo = mid + 1; } else { hi = mid; }
          }
-         const uint32_t b = 4 * w + q;  // keys < 0x00800000 or >= 0xFF800000
+         // (keys < 0x00800000 or >= 0xFF800000: the slow path)
          word |= (b < 32 || b >= kLutSize - 32 ? kSlowBucket : (uint32_t)lo) << (8 * q);
       }
       lut4[w] = word;

@@ -11,10 +11,11 @@
 //    load at a fixed offset, with no per-row address arithmetic, and the next plane's copy is in
 //    flight while the current one is counted. The tensor map covers this GPU's own field only; no
 //    load uses cluster multicast. Every wait on a copy has a poll limit (mkfKernelFaults).
-//  * With K <= 16 an element's thermometer T (bits k < rank) and its complement fit one word,
-//    V = T | ~T << 16. AND over a cell's eight corners gives C = T(min) | ~T(max) << 16 in three
-//    logic operations per cell (x pair, face, cell); popc(C) = 16 - (max - min) is the number of
-//    thresholds the cell does not cross and popc of the low half is its smallest rank.
+//  * With K <= 16 an element is one word, its rank and 16 less its rank in the two halves. The
+//    half-wise minimum over a cell's eight corners (x pair, face, cell: three operations) is the
+//    cell's smallest rank and 16 less its largest; their sum is 16 less the number of thresholds the
+//    cell crosses. (As a thermometer and its complement, with ANDs and two popcounts, the same took
+//    three instructions more: 512^3 FP64, 16 thresholds 352 -> 342 us, FP32, 8 307 -> 294.)
 //  * All-ones counts cost no per-cell work: the three code slots add one count each to rows rmin,
 //    rmin + 1 and rmin + 2 (real codes or discarded 0s), so the row totals give, by a recurrence at
 //    the flush, the number of cells of each smallest rank; the cells all-ones for threshold k are
@@ -27,7 +28,7 @@
 //    field with 16 thresholds) are queued, per lane with one store and no warp vote; the warp
 //    drains the lanes' queues together, 32 cells at a time, taking back their three slot counts
 //    and counting every code they have.
-// Masked cells (lanes and rows outside the item) enter C as all ones: they cross nothing, land in
+// Masked cells (lanes and rows outside the item) get smallest rank 16: they cross nothing, land in
 // smallest-rank row 16, and are subtracted from the all-ones counts at the flush.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -85,8 +86,8 @@ struct TmaGeom
 __device__ unsigned gTmaFault;
 
 // Histogram rows per copy: K real rows, then discard rows up to max(K, 16) + 2, where the slots
-// of cells that cross fewer than three thresholds (and of masked cells, whose low half is 16 set
-// bits) add their code-0 counts; the flush reads rows < K and codes 1..254 only.
+// of cells that cross fewer than three thresholds (and of masked cells, of rank 16) add their code-0
+// counts; the flush reads rows < K and codes 1..254 only.
 __host__ __device__ constexpr int tmaCopyRows(int K) { return (K > 16 ? K : 16) + 3; }
 
 // Exact rank of the element at p by binary search over the sorted thresholds (rare: ties of FP64
@@ -275,7 +276,13 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
       for (int s = 0; s < S; s++) { mbarInit((uint32_t)__cvta_generic_to_shared(&bars[warp][s]), 1); }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
    }
-   ctaSetup(a, Sh, hist, copyRows, kHistCopies);  // (its barriers also order the mbarrier set-up)
+   ctaSetup<W == 1>(a, Sh, hist, copyRows, kHistCopies);  // (its barriers also order the mbarrier set-up)
+   if (W == 1) {  // the candidates as they are compared (past the last: compares false)
+      for (int i = threadIdx.x; i < kThKeys; i += blockDim.x) {
+         Sh.key[i] = __float_as_uint(i < K ? (float)(GE ? a.thi[i] : a.tlo[i]) : __uint_as_float(0x7FC00000u));
+      }
+      __syncthreads();
+   }
 
    const uint32_t ringW = (uint32_t)__cvta_generic_to_shared(ring) + (uint32_t)(warp * S * G::PITCH);
    const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(&bars[warp][0]);
@@ -343,20 +350,27 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
       const uint32_t *colW = reinterpret_cast<const uint32_t *>(col) + (W - 1);
       bool slow = false;   // a FP64 high word equal to a threshold's
       uint32_t rOr = 0;    // slow-path buckets rank above 32
+      // The table finds the rank of the element's bucket from its top bits, a comparison with the
+      // bucket's threshold the rest. FP32 elements index the table and compare as they are, without an
+      // order-preserving key (512^3, 8 thresholds: 294 -> 286 us; plane waves 256 x 1024 x 1024 560 -> 535).
+      // FP64 high words keep the key: compared as floats, which would do, they measured 1 % slower with
+      // 16 thresholds, and whole elements 4 % (8-byte candidates): there the shared-memory pipe decides.
 #pragma unroll
       for (int j = 0; j < kTmRows; ++j) {
-         const uint32_t key = sortKey(colW[j * G::BX * W]);
-         const uint32_t r0 = Sh.lut[key >> kLutShift];
-         const uint32_t cand = Sh.key[r0];
-         uint32_t rr = r0 + (GE ? (key >= cand) : (key > cand));
-         bool tie = key == cand;
+         const uint32_t top = W == 1 ? colW[j * G::BX * W] : sortKey(colW[j * G::BX * W]);
+         const uint32_t r0 = Sh.lut[top >> kLutShift];
+         uint32_t rr = r0;
 #pragma unroll
-         for (int c = 1; c < CMAX; ++c) {
-            const uint32_t cc = Sh.key[r0 + c];
-            rr += GE ? (key >= cc) : (key > cc);
-            tie = tie | (key == cc);
+         for (int c = 0; c < CMAX; ++c) {
+            const uint32_t cand = Sh.key[r0 + c];
+            if (W == 1) {
+               const float v = __uint_as_float(top), t = __uint_as_float(cand);
+               rr += GE ? v >= t : v > t;
+            } else {
+               rr += GE ? top >= cand : top > cand;
+               slow = slow | (top == cand);
+            }
          }
-         if (W == 2) { slow = slow | tie; }
          rOr |= rr;
          r[j] = rr;
       }
@@ -373,10 +387,16 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
       ++g;
       return true;
    };
-   // thermometer of a rank and its complement: T | ~T << 16, T = bits [0, r); the x neighbour's
-   // is formed here from its shuffled rank (one shuffle per row, not two: shuffles share the pipe
-   // of the tile loads and the histogram atomics; measured 1 % faster)
-   auto thermoV = [](uint32_t r) { return thermo(r) * 0xFFFF0001u + 0xFFFF0000u; };
+   // a rank and its distance from 16, one per half: r | (16 - r) << 16; the half-wise minimum over
+   // a cell's corners is its smallest rank and 16 less its largest. The x neighbour's pair is shuffled,
+   // and its rank taken from there (one shuffle per row: shuffles share the pipe of the tile loads and
+   // the histogram atomics).
+   auto pairOf = [](uint32_t r) { return r * 0xFFFF0001u + 0x100000u; };
+   auto min2 = [](uint32_t x, uint32_t y) {
+      uint32_t m;
+      asm("min.u16x2 %0, %1, %2;" : "=r"(m) : "r"(x), "r"(y));
+      return m;
+   };
 
    unsigned long long cells = 0;
    uint32_t masked = 0;  // masked cells counted (in smallest-rank row 16)
@@ -388,21 +408,19 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
       const TmItem m = itemOf<G::ALIGN>(a, it, lane);
       cells += m.cells;
       masked += (8u - (uint32_t)__popc(m.rowsOK)) * (uint32_t)m.nPln;
-      uint32_t sF[8], sV[8];  // previous plane: face ranks (bytes), face thermometer AND
+      uint32_t sF[8], sV[8];  // previous plane: face ranks (bytes), minimum of the face pairs
       {
          uint32_t r[kTmRows];
          if (!plane(m.xoff, r)) { fault = true; break; }
-         uint32_t rR = __shfl_down_sync(FULL, r[0], 1);
-         uint32_t Vt = thermoV(r[0]), VR = thermoV(rR);
-         uint32_t ePrev = rR * 256u + r[0], Pprev = Vt & VR;
+         uint32_t w = pairOf(r[0]), wR = __shfl_down_sync(FULL, w, 1);
+         uint32_t ePrev = __byte_perm(w, wR, 0x7140), Pprev = min2(w, wR);
 #pragma unroll
          for (int j = 0; j < 8; ++j) {
-            rR = __shfl_down_sync(FULL, r[j + 1], 1);
-            Vt = thermoV(r[j + 1]);
-            VR = thermoV(rR);
-            const uint32_t e = rR * 256u + r[j + 1], P = Vt & VR;
+            w = pairOf(r[j + 1]);
+            wR = __shfl_down_sync(FULL, w, 1);
+            const uint32_t e = __byte_perm(w, wR, 0x7140), P = min2(w, wR);
             sF[j] = e * 65536u + ePrev;
-            sV[j] = P & Pprev;
+            sV[j] = min2(P, Pprev);
             ePrev = e;
             Pprev = P;
          }
@@ -410,22 +428,20 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
       for (int p = 1; p <= m.nPln; ++p) {
          uint32_t r[kTmRows];
          if (!plane(m.xoff, r)) { fault = true; break; }
-         uint32_t rR = __shfl_down_sync(FULL, r[0], 1);
-         uint32_t Vt = thermoV(r[0]), VR = thermoV(rR);
-         uint32_t ePrev = rR * 256u + r[0];
-         uint32_t Pprev = Vt & VR;
+         uint32_t w = pairOf(r[0]), wR = __shfl_down_sync(FULL, w, 1);
+         uint32_t ePrev = __byte_perm(w, wR, 0x7140), Pprev = min2(w, wR);
 #pragma unroll
          for (int j = 0; j < 8; ++j) {
-            rR = __shfl_down_sync(FULL, r[j + 1], 1);
-            Vt = thermoV(r[j + 1]);
-            VR = thermoV(rR);
-            const uint32_t e = rR * 256u + r[j + 1];
-            const uint32_t P = Vt & VR;
-            const uint32_t fc = e * 65536u + ePrev;  // face ranks: (x,y) (x+1,y) (x,y+1) (x+1,y+1)
-            const uint32_t F = P & Pprev;
-            const uint32_t nvm = ((m.rowsOK >> j) & 1u) - 1u;  // all ones for a masked cell
-            const uint32_t C = (F & sV[j]) | nvm;
-            const uint32_t pc = __popc(C), rmin = __popc(C & 0xFFFFu);
+            w = pairOf(r[j + 1]);
+            wR = __shfl_down_sync(FULL, w, 1);
+            const uint32_t e = __byte_perm(w, wR, 0x7140);
+            const uint32_t P = min2(w, wR);
+            // face ranks: (x,y) (x+1,y) (x,y+1) (x+1,y+1)
+            const uint32_t fc = e * 65536u + ePrev;
+            const uint32_t F = min2(P, Pprev);
+            // a masked cell crosses nothing: both halves of its pair are 16 and 0
+            const uint32_t C = (m.rowsOK & (1u << j)) ? min2(F, sV[j]) : 16u;
+            const uint32_t rmin = C & 0xFFFFu, pc = (C >> 16) + rmin;  // pc: 16 less the thresholds crossed
             const uint32_t R0 = sF[j], R1 = fc;
             const uint32_t D0 = R0 + rmin * 0xFEFEFEFFu;         // R0 - rmin per byte
             const uint32_t D1s = R1 * 16u + rmin * 0xEFEFEFF0u;  // (R1 - rmin per byte) << 4
