@@ -142,14 +142,16 @@ struct CountArgs
    int X;                  // elements per row
    int rows, planes;       // row pairs + 1, plane pairs + 1
    uint32_t rowWS, planeWS;
-   long long nItems;       // rowWS * (rows-1) * (planes-1)
+   long long nItems;       // rowWS * (rows-1) * runs of kCountZ plane pairs
    unsigned long long *out;
 };
 
-// Packed map -> 256 counts. Each thread takes 32 cells of one row pair of one plane pair: the
-// four row words and their successors give eight 32-bit corner masks v0..v7 (bit j = corner i of
-// cell x = 32w + j). Uniform cells (all corners equal) are counted by popcount; only mixed cells
-// form their 8-bit code, counted in a per-warp shared histogram.
+// Packed map -> 256 counts. Each thread takes 32 cells of one row pair in kCountZ plane pairs, all of
+// its map words loaded before the first is used (the kernel is bound by the latency of these loads:
+// one plane pair at a time, four in turn per thread, took 11.9 us for the 256^3 map under ncu, this
+// 9.5). A cell's corners are bits b and b + 1 of four words; uniform cells (all corners equal) are
+// counted by popcount; only mixed cells form their 8-bit code, counted in a per-warp shared histogram.
+static constexpr int kCountZ = 4;
 template <typename I>
 __global__ void __launch_bounds__(256) countMap(const __grid_constant__ CountArgs a)
 {
@@ -168,32 +170,43 @@ __global__ void __launch_bounds__(256) countMap(const __grid_constant__ CountArg
       const int wi = (int)(i - rp * rowWS);
       const I zq = rp / rowPairs;
       const int y = (int)(rp - zq * rowPairs);
-      const int z = (int)zq;
+      const int z = (int)zq * kCountZ, nZ = min(kCountZ, a.planes - 1 - z);
       const int nValid = min(32, a.X - 1 - 32 * wi);
       if (nValid <= 0) { continue; }
       const uint32_t vmask = (nValid >= 32) ? 0xFFFFFFFFu : ((1u << nValid) - 1u);
-      const uint32_t *p0 = a.w + (size_t)z * a.planeWS + (size_t)y * a.rowWS + wi;
-      const uint32_t *p1 = p0 + a.planeWS;
       const bool nx = (wi + 1) < (int)a.rowWS;
-      const uint32_t r0 = p0[0], r1 = p0[a.rowWS], r2 = p1[0], r3 = p1[a.rowWS];
-      const uint32_t n0w = nx ? p0[1] : 0u, n1w = nx ? p0[a.rowWS + 1] : 0u;
-      const uint32_t n2w = nx ? p1[1] : 0u, n3w = nx ? p1[a.rowWS + 1] : 0u;
-      const uint32_t v0 = r0, v1 = __funnelshift_r(r0, n0w, 1);
-      const uint32_t v2 = r1, v3 = __funnelshift_r(r1, n1w, 1);
-      const uint32_t v4 = r2, v5 = __funnelshift_r(r2, n2w, 1);
-      const uint32_t v6 = r3, v7 = __funnelshift_r(r3, n3w, 1);
-      const uint32_t all = v0 & v1 & v2 & v3 & v4 & v5 & v6 & v7 & vmask;
-      const uint32_t none = ~(v0 | v1 | v2 | v3 | v4 | v5 | v6 | v7) & vmask;
-      uint32_t mixed = vmask & ~(all | none);
-      n255 += __popc(all);
-      n0 += __popc(none);
-      while (mixed) {
-         const int j = __ffs(mixed) - 1;
-         mixed &= mixed - 1;
-         const uint32_t c = ((v0 >> j) & 1u) | (((v1 >> j) & 1u) << 1) | (((v2 >> j) & 1u) << 2) |
-                            (((v3 >> j) & 1u) << 3) | (((v4 >> j) & 1u) << 4) | (((v5 >> j) & 1u) << 5) |
-                            (((v6 >> j) & 1u) << 6) | (((v7 >> j) & 1u) << 7);
-         atomicAdd(h + c, 1u);
+      // per plane: the two rows' words and the words after them (bit 0 is used)
+      uint32_t w[kCountZ + 1][4];
+#pragma unroll
+      for (int p = 0; p <= kCountZ; p++) {
+         const uint32_t *q = a.w + (size_t)(z + min(p, nZ)) * a.planeWS + (size_t)y * a.rowWS + wi;
+         w[p][0] = q[0];
+         w[p][1] = q[a.rowWS];
+         w[p][2] = nx ? q[1] : 0u;
+         w[p][3] = nx ? q[a.rowWS + 1] : 0u;
+      }
+#pragma unroll
+      for (int p = 0; p < kCountZ; p++) {
+         const uint32_t v0 = w[p][0], v2 = w[p][1], v4 = w[p + 1][0], v6 = w[p + 1][1];
+         const uint32_t v1 = __funnelshift_r(v0, w[p][2], 1), v3 = __funnelshift_r(v2, w[p][3], 1);
+         const uint32_t v5 = __funnelshift_r(v4, w[p + 1][2], 1), v7 = __funnelshift_r(v6, w[p + 1][3], 1);
+         const uint32_t vm = p < nZ ? vmask : 0u;
+         const uint32_t all = v0 & v1 & v2 & v3 & v4 & v5 & v6 & v7 & vm;
+         const uint32_t none = ~(v0 | v1 | v2 | v3 | v4 | v5 | v6 | v7) & vm;
+         uint32_t mixed = vm & ~(all | none);
+         n255 += __popc(all);
+         n0 += __popc(none);
+         // word j's bits b, b + 1 go to code bits 2j, 2j + 1: shifted left by 2j as a (hi:lo) pair, the
+         // top bit from the x + 1 word, one funnel shift by b brings them into place
+         const uint32_t l1 = v2 << 2, h1 = v3 >> 29, l2 = v4 << 4, h2 = v5 >> 27, l3 = v6 << 6, h3 = v7 >> 25;
+         while (mixed) {
+            const int j = 31 - __clz(mixed);
+            mixed ^= 1u << j;
+            uint32_t c = (__funnelshift_r(l1, h1, j) & ~3u) | (__funnelshift_r(v0, v1 >> 31, j) & 3u);
+            c = (__funnelshift_r(l2, h2, j) & ~15u) | (c & 15u);
+            c = (__funnelshift_r(l3, h3, j) & ~63u) | (c & 63u);
+            atomicAdd(h + (c & 255u), 1u);
+         }
       }
    }
    n0 = __reduce_add_sync(FULL, (unsigned)n0) ;
@@ -223,10 +236,10 @@ static int launchCount(unsigned long long *out, const BMOrg *pO, const uint32_t 
    a.planeWS = pO->planeWS;
    a.out = out;
    if (pO->rowPairs == 0 || pO->planePairs == 0 || pO->rowElem < 2 || pO->rowWS == 0) { return MKF_OK; }
-   a.nItems = (long long)a.rowWS * pO->rowPairs * pO->planePairs;
-   // at least 4 words per thread, at most 4 CTAs per SM: every CTA ends with up to 256 global
-   // atomics on the same 256 counters, so fewer, busier CTAs finish sooner
-   long long grid = (a.nItems + 1023) / 1024;
+   a.nItems = (long long)a.rowWS * pO->rowPairs * ((pO->planePairs + kCountZ - 1) / kCountZ);
+   // one item per thread up to 4 CTAs per SM: every CTA ends with up to 256 global atomics on the same
+   // 256 counters, so fewer, busier CTAs finish sooner
+   long long grid = (a.nItems + 255) / 256;
    const long long cap = (long long)smCount() * 4;
    if (grid > cap) { grid = cap; }
    if (grid < 1) { grid = 1; }
