@@ -57,14 +57,12 @@ def _enc_of(t) -> int:
 
 def _field_desc(ptr: int, enc: int, shape_zyx, strides_zyx=None) -> MKFFieldDesc:
     """Descriptor of a (Z, Y, X) field; strides in elements (None = planar)."""
-    d = MKFFieldDesc()
-    d.p = ptr
-    d.enc = enc
-    z, y, x = (int(v) for v in shape_zyx)
-    d.def_[0], d.def_[1], d.def_[2] = x, y, z
+    d = MKFFieldDesc(ptr, enc)
+    v = d.def_
+    v[2], v[1], v[0] = shape_zyx
     if strides_zyx is not None:
-        sz, sy, sx = (int(v) for v in strides_zyx)
-        d.stride[0], d.stride[1], d.stride[2] = sx, sy, sz
+        v = d.stride
+        v[2], v[1], v[0] = strides_zyx
     return d
 
 
@@ -72,21 +70,21 @@ class _Thresholds:
     """Keeps the ctypes arrays of a threshold set alive while a call uses them."""
 
     def __init__(self, t, m):
-        t = np.atleast_1d(np.asarray(t, np.float64))
-        self.t = (C.c_double * t.size)(*t.tolist())
-        ts = MKFThreshSet()
-        ts.nT = t.size
-        if np.ndim(m) == 0:
-            ts.mAll = int(m)
-            ts.m = None
-            self.m = None
+        shape = None
+        if type(t) is not list or not all(type(v) is float for v in t):
+            t = np.atleast_1d(np.asarray(t, np.float64))
+            shape = t.shape
+            t = t.tolist()
+        n = len(t)
+        self.t = (C.c_double * n)(*t)
+        self.m = None
+        if type(m) is int or np.ndim(m) == 0:
+            self.ts = MKFThreshSet(n, int(m), self.t, None)
         else:
-            mm = np.broadcast_to(np.asarray(m, np.uint32), t.shape)
-            self.m = (C.c_uint32 * t.size)(*mm.tolist())
-            ts.m = C.cast(self.m, C.POINTER(C.c_uint32))
-        ts.t = C.cast(self.t, C.POINTER(C.c_double))
-        self.ts = ts
-        self.n = t.size
+            mm = np.broadcast_to(np.asarray(m, np.uint32), shape or (n,))
+            self.m = (C.c_uint32 * n)(*mm.tolist())
+            self.ts = MKFThreshSet(n, 0, self.t, self.m)
+        self.n = n
 
 
 def _stream_ptr(stream) -> int | None:
@@ -102,8 +100,8 @@ def field_bpfd(field, thresholds, mask=BMC_GT, out=None, accumulate=False, strea
     Returns (or fills) a uint64-valued int64 CUDA tensor of shape (K, 256)."""
     torch = _torch()
     th = _Thresholds(thresholds, mask)
-    if out is None:
-        out = torch.zeros((th.n, 256), dtype=torch.int64, device=field.device)
+    if out is None:  # (cleared by the call unless it accumulates)
+        out = (torch.zeros if accumulate else torch.empty)((th.n, 256), dtype=torch.int64, device=field.device)
     strides = None if field.is_contiguous() else field.stride()
     d = _field_desc(field.data_ptr(), _enc_of(field), field.shape, strides)
     rc = lib().mkfFieldBPFD(out.data_ptr(), C.byref(d), C.byref(th.ts),
@@ -118,8 +116,8 @@ def field_bpfd_moments(field, thresholds, mask=BMC_GT, stream=None):
     moments (K, 2, 2) float64), both CUDA tensors."""
     torch = _torch()
     th = _Thresholds(thresholds, mask)
-    out = torch.zeros((th.n, 256), dtype=torch.int64, device=field.device)
-    mom = torch.zeros((th.n, 2, 2), dtype=torch.float64, device=field.device)
+    out = torch.empty((th.n, 256), dtype=torch.int64, device=field.device)  # (both cleared by the call)
+    mom = torch.empty((th.n, 2, 2), dtype=torch.float64, device=field.device)
     strides = None if field.is_contiguous() else field.stride()
     d = _field_desc(field.data_ptr(), _enc_of(field), field.shape, strides)
     check(lib().mkfFieldBPFDMoments(out.data_ptr(), mom.data_ptr(), C.byref(d), C.byref(th.ts), 0, _stream_ptr(stream)),

@@ -254,17 +254,47 @@ static size_t gMapWords = 0;
 static size_t *gBPFDDev = nullptr;
 static size_t *gBPFDHost = nullptr;
 
-struct EventTimer
+static size_t *gBPFDStage = nullptr;  // pinned: counts on their way to the caller's array
+
+// Stage timer of the original's interface. The two events belong to the calling thread and device and
+// are kept between calls (creating and destroying them cost 4 us of each call).
+class EventTimer
 {
-   cudaEvent_t e0 = nullptr, e1 = nullptr;
-   EventTimer() { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, 0); }
-   ~EventTimer() { cudaEventDestroy(e0); cudaEventDestroy(e1); }
-   float stop() {
+ public:
+   EventTimer() { cudaEventRecord(ev().e0, 0); }
+   void mark() { cudaEventRecord(ev().e1, 0); }
+   // wait for the mark (or for work issued after it on the stream: one wait for both) and read the time
+   float stop(bool stream = false) {
       float ms = 0;
-      cudaEventRecord(e1, 0);
-      cudaEventSynchronize(e1);
-      cudaEventElapsedTime(&ms, e0, e1);
+      if (stream) { cudaStreamSynchronize(0); }
+      else { cudaEventSynchronize(ev().e1); }
+      cudaEventElapsedTime(&ms, ev().e0, ev().e1);
       return ms;
+   }
+
+ private:
+   struct Events
+   {
+      int dev = -1;
+      cudaEvent_t e0 = nullptr, e1 = nullptr;
+      void drop() {
+         if (e0) { cudaEventDestroy(e0); }
+         if (e1) { cudaEventDestroy(e1); }
+         e0 = e1 = nullptr;
+      }
+      ~Events() { drop(); }
+   };
+   static Events &ev() {
+      static thread_local Events e;
+      int dev = 0;
+      cudaGetDevice(&dev);
+      if (e.dev != dev || !e.e0 || !e.e1) {
+         e.drop();
+         cudaEventCreate(&e.e0);
+         cudaEventCreate(&e.e1);
+         e.dev = dev;
+      }
+      return e;
    }
 };
 
@@ -340,6 +370,7 @@ MKF_API BMPackWord *binMapCUDA(KernInfo *pK, BMPackWord *pW, BMOrg *pO, const BM
    if (pF->elemID == ENC_F32) { launchPack<float>(a, grid); }
    else { launchPack<double>(a, grid); }
    cudaError_t e = cudaGetLastError();
+   tm.mark();
    const float ms = tm.stop();
    if (e == cudaSuccess) { e = cudaGetLastError(); }
    if (e != cudaSuccess) {
@@ -362,6 +393,7 @@ MKF_API size_t *mkfCUDAGetBPFD(KernInfo *pK, size_t *pBPFD, const BMOrg *pO, con
    if (!pO || !pW) { return pBPFD; }
    EventTimer tm;
    const int rc = launchCount((unsigned long long *)pBPFD, pO, pW, 0);
+   tm.mark();
    const float ms = tm.stop();
    if (rc != MKF_OK) { logError("mkfCUDAGetBPFD() - %s\n", mkfLastError()); }
    if (pK) { pK->dtms[1] = ms; }
@@ -370,18 +402,28 @@ MKF_API size_t *mkfCUDAGetBPFD(KernInfo *pK, size_t *pBPFD, const BMOrg *pO, con
 
 MKF_API size_t *mkfCUDAGetBPFDH(KernInfo *pK, size_t *pBPFDH, const BMOrg *pO, const BMPackWord *pW, const int profile)
 {
+   (void)profile;
    const size_t bytes = sizeof(size_t) * MKF_BINS;
    if (!pBPFDH) {
       if (!gBPFDHost && cudaMallocHost(&gBPFDHost, bytes) != cudaSuccess) { cudaGetLastError(); gBPFDHost = nullptr; }
       pBPFDH = gBPFDHost;
    }
    if (!gBPFDDev && cudaMalloc(&gBPFDDev, bytes) != cudaSuccess) { cudaGetLastError(); gBPFDDev = nullptr; }
-   if (!pBPFDH || !gBPFDDev) { return nullptr; }
-   cudaMemset(gBPFDDev, 0, bytes);
+   if (!gBPFDStage && cudaMallocHost(&gBPFDStage, bytes) != cudaSuccess) { cudaGetLastError(); gBPFDStage = nullptr; }
+   if (!pBPFDH || !gBPFDDev || !gBPFDStage) { return nullptr; }
+   cudaMemsetAsync(gBPFDDev, 0, bytes, 0);
    cudaGetLastError();  // clear any error left by earlier calls before checking ours
-   if (!mkfCUDAGetBPFD(pK, gBPFDDev, pO, pW, profile)) { return nullptr; }
-   const cudaError_t e = cudaMemcpy(pBPFDH, gBPFDDev, bytes, cudaMemcpyDeviceToHost);
+   // the count and the copy of its result in one go, with one wait at the end
+   EventTimer tm;
+   const int rc = (pO && pW) ? launchCount((unsigned long long *)gBPFDDev, pO, pW, 0) : MKF_OK;
+   tm.mark();
+   cudaError_t e = cudaMemcpyAsync(gBPFDStage, gBPFDDev, bytes, cudaMemcpyDeviceToHost, 0);
+   const float ms = tm.stop(true);
+   if (rc != MKF_OK) { logError("mkfCUDAGetBPFD() - %s\n", mkfLastError()); }
+   if (pK && pO && pW) { pK->dtms[1] = ms; }
+   if (e == cudaSuccess) { e = cudaGetLastError(); }
    if (e != cudaSuccess) { logError("mkfCUDAGetBPFDH() - r=%d -> %s\n", (int)e, cudaGetErrorName(e)); return nullptr; }
+   memcpy(pBPFDH, gBPFDStage, bytes);
    return pBPFDH;
 }
 
@@ -390,6 +432,7 @@ MKF_API void mkfCUDACleanup(int lvl)
    (void)lvl;  // the original resets the device when lvl > 0; a shared device is never reset here
    if (gBPFDHost) { cudaFreeHost(gBPFDHost); gBPFDHost = nullptr; }
    if (gBPFDDev) { cudaFree(gBPFDDev); gBPFDDev = nullptr; }
+   if (gBPFDStage) { cudaFreeHost(gBPFDStage); gBPFDStage = nullptr; }
 }
 
 MKF_API int mkfCUDAGetBPFDautoCtx(Context *pC, const FieldDef def[3], const BinMapF64 *pM, const int profile)
