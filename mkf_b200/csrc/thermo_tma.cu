@@ -16,17 +16,17 @@
 //    cell's smallest rank and 16 less its largest; their sum is 16 less the number of thresholds the
 //    cell crosses. (As a thermometer and its complement, with ANDs and two popcounts, the same took
 //    three instructions more: 512^3 FP64, 16 thresholds 352 -> 342 us, FP32, 8 307 -> 294.)
-//  * All-ones counts cost no per-cell work: the three code slots add one count each to rows rmin,
-//    rmin + 1 and rmin + 2 (real codes or discarded 0s), so the row totals give, by a recurrence at
-//    the flush, the number of cells of each smallest rank; the cells all-ones for threshold k are
-//    those whose smallest rank exceeds k.
+//  * All-ones counts cost no per-cell work: the three code slots (two with few thresholds, twoSlots)
+//    add one count each to rows rmin, rmin + 1 and rmin + 2 (real codes or discarded 0s), so the row
+//    totals give, by a recurrence at the flush, the number of cells of each smallest rank; the cells
+//    all-ones for threshold k are those whose smallest rank exceeds k.
 //  * Mixed codes for k = min, min + 1, min + 2 come from two bit-planes of the corner ranks
 //    relative to min; each goes to the shared [K][257] histogram with an unpredicated atomic whose
 //    address is the code's top byte masked in place plus the row. Where the cell crosses q or
 //    fewer thresholds the code of slot q is 0, and those counts land in bins the flush skips (and
-//    in discard rows past K). Cells crossing four or more thresholds (about 1 in 100 on a smooth
+//    in discard rows past K). Cells crossing more thresholds than slots (about 1 in 100 on a smooth
 //    field with 16 thresholds) are queued, per lane with one store and no warp vote; the warp
-//    drains the lanes' queues together, 32 cells at a time, taking back their three slot counts
+//    drains the lanes' queues together, 32 cells at a time, taking back their slot counts
 //    and counting every code they have.
 // Masked cells (lanes and rows outside the item) get smallest rank 16: they cross nothing, land in
 // smallest-rank row 16, and are subtracted from the all-ones counts at the flush.
@@ -118,12 +118,13 @@ __device__ __forceinline__ uint32_t codeAddr(uint32_t c, uint32_t base)
    return a;
 }
 
-// Count the queued wide cells (spread >= 4) of a warp: lane i takes entries i, i + 32, ...; an
+// Count the queued wide cells (spread > NS) of a warp: lane i takes entries i, i + 32, ...; an
 // entry is the cell's two faces of corner ranks (bytes), its smallest rank and spread follow from
-// them. The row loop added three codes for each of them from two rank bit-planes, which are wrong
+// them. The row loop added NS codes for each of them from two rank bit-planes, which are wrong
 // past a spread of 3; they are taken back here (the same formulas, minus one), then every code
 // k = rmin .. rmax - 1 is counted: fixed formulas up to a spread of 7, one threshold at a time
 // beyond (thermo.cu counts them the same way).
+template <int NS>
 __device__ __forceinline__ void wideCell(const uint2 e, uint32_t hist32)
 {
    {
@@ -146,7 +147,7 @@ __device__ __forceinline__ void wideCell(const uint2 e, uint32_t hist32)
          const uint32_t a2 = codeAddr((G0 & G1) & 0xFF000000u, rowAddr);
          asm volatile("red.shared.add.u32 [%0], -1;" ::"r"(a0) : "memory");
          asm volatile("red.shared.add.u32 [%0+%1], -1;" ::"r"(a1), "n"(kHistRow * 4) : "memory");
-         asm volatile("red.shared.add.u32 [%0+%1], -1;" ::"r"(a2), "n"(kHistRow * 8) : "memory");
+         if (NS == 3) { asm volatile("red.shared.add.u32 [%0+%1], -1;" ::"r"(a2), "n"(kHistRow * 8) : "memory"); }
       }
       if (spread < 8) {
          const uint32_t b0 = gatherBits((D0 & 0x01010101u) | (D1s & 0x10101010u), 0x01020408u);
@@ -155,7 +156,7 @@ __device__ __forceinline__ void wideCell(const uint2 e, uint32_t hist32)
          redSharedAt<0>((b0 | b1 | b2) * 4u + rowAddr);
          redSharedAt<kHistRow * 4>((b1 | b2) * 4u + rowAddr);
          redSharedAt<kHistRow * 8>((b2 | (b1 & b0)) * 4u + rowAddr);
-         redSharedAt<kHistRow * 12>(b2 * 4u + rowAddr);
+         if (NS == 3 || spread > 3) { redSharedAt<kHistRow * 12>(b2 * 4u + rowAddr); }
          if (spread > 4) { redSharedAt<kHistRow * 16>((b2 & (b1 | b0)) * 4u + rowAddr); }
          if (spread > 5) { redSharedAt<kHistRow * 20>((b2 & b1) * 4u + rowAddr); }
          if (spread > 6) { redSharedAt<kHistRow * 24>((b2 & b1 & b0) * 4u + rowAddr); }
@@ -167,19 +168,20 @@ __device__ __forceinline__ void wideCell(const uint2 e, uint32_t hist32)
             addr += kHistRow * 4;
          }
       }
-      // row totals count every cell once in rows rmin .. rmin + 2: take back the codes counted in
-      // rows rmin + 3 .. rmax - 1 from those rows' spare word
-      for (uint32_t q = 3; q < spread; ++q) {
+      // row totals count every cell once in rows rmin .. rmin + NS - 1: take back the codes counted in
+      // rows rmin + NS .. rmax - 1 from those rows' spare word
+      for (uint32_t q = NS; q < spread; ++q) {
          asm volatile("red.shared.add.u32 [%0+%1], -1;" ::"r"(rowAddr + q * (kHistRow * 4)), "n"(256 * 4) : "memory");
       }
    }
 }
 
 // Drain a warp's queue of n entries: lane i takes entries i, i + 32, ...
+template <int NS>
 __device__ __noinline__ void drainWide(const uint2 *q, int n, uint32_t hist32)
 {
    __syncwarp();
-   for (int i = threadIdx.x & 31; i < n; i += 32) { wideCell(q[i], hist32); }
+   for (int i = threadIdx.x & 31; i < n; i += 32) { wideCell<NS>(q[i], hist32); }
    __syncwarp();
 }
 
@@ -187,6 +189,7 @@ __device__ __noinline__ void drainWide(const uint2 *q, int n, uint32_t hist32)
 // q * 32 + l; n: this lane's entries), 32 entries per round whatever their owners: entry g of the
 // warp (in lane order) belongs to the last lane whose exclusive prefix of counts is <= g, found
 // by a binary search over the lanes' prefixes. Inline (measured 1 % faster than a call).
+template <int NS>
 __device__ __forceinline__ void drainLanes(const uint2 *qw, int n, uint32_t hist32)
 {
    __syncwarp();  // (orders the other lanes' queue stores before these loads)
@@ -207,7 +210,7 @@ __device__ __forceinline__ void drainLanes(const uint2 *qw, int n, uint32_t hist
          if (e <= g) { owner += s; }
       }
       const int q = g - __shfl_sync(FULL, excl, owner);
-      if (g < total) { wideCell(qw[32 * q + owner], hist32); }
+      if (g < total) { wideCell<NS>(qw[32 * q + owner], hist32); }
    }
    __syncwarp();
 }
@@ -249,7 +252,7 @@ __device__ __forceinline__ TmItem itemOf(const FusedArgs &a, long long it, int l
 // waits for its own copies only; the rest is the same. Against thermo.cu, which took these fields
 // before (B200, us): 333 x 401 x 487 FP64, 12 thresholds 240 -> 197, 16 265 -> 212; 301 x 333 x 277 FP32, 8
 // 110 -> 77; 100 x 101 x 99 FP64, 12 27 -> 18.
-template <typename T, bool GE, int CMAX, int V, bool TMA>
+template <typename T, bool GE, int CMAX, int V, bool TMA, int NS>
 __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
     thermoTmaBPFD(const __grid_constant__ FusedArgs a, const __grid_constant__ CUtensorMap tm)
 {
@@ -456,23 +459,23 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
             // such counts land in discard bins
             redSharedAt<0>(codeAddr((G0 | G1) & 0xFF000000u, rowAddr));
             redSharedAt<kHistRow * 4>(codeAddr(G1 & 0xFF000000u, rowAddr));
-            redSharedAt<kHistRow * 8>(codeAddr((G0 & G1) & 0xFF000000u, rowAddr));
-            // cells crossing 4 or more thresholds join the queue
+            if (NS == 3) { redSharedAt<kHistRow * 8>(codeAddr((G0 & G1) & 0xFF000000u, rowAddr)); }
+            // cells crossing more thresholds join the queue
             if (G::LANEQ) {
                // a predicated 64-bit store and a predicated advance, no branch (measured against
                // two 32-bit stores: 2 % faster; against skipping the stores when no lane of the
                // warp has a wide cell: 3-4 % faster, even with 8 thresholds where none has)
                asm volatile(
                    "{\n\t.reg .pred w;\n\t"
-                   "setp.lt.u32 w, %1, 13;\n\t"
+                   "setp.lt.u32 w, %1, %4;\n\t"
                    "@w st.shared.v2.u32 [%0], {%2, %3};\n\t"
                    "@w add.u32 %0, %0, 256;\n\t}"
                    : "+r"(qa)
-                   : "r"(pc), "r"(R0), "r"(R1)
+                   : "r"(pc), "r"(R0), "r"(R1), "n"(16 - NS)
                    : "memory");
             } else {
                // every lane stores (the others into the discard entry), so the row body has no branch
-               const bool wide = pc < 13u;
+               const bool wide = pc < (uint32_t)(16 - NS);
                const uint32_t wb = __ballot_sync(FULL, wide);
                queue[wide ? qn + __popc(wb & lanesBelow) : kTmQueue] = make_uint2(R0, R1);
                qn += __popc(wb);
@@ -484,11 +487,11 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
          }
          if (G::LANEQ) {
             if (__any_sync(FULL, qa > qLane0 + (kTmLaneQ - 8) * 256u)) {
-               drainLanes(queue, (int)((qa - qLane0) >> 8), hist32);
+               drainLanes<NS>(queue, (int)((qa - qLane0) >> 8), hist32);
                qa = qLane0;
             }
          } else if (qn >= 32) {
-            drainWide(queue, qn, hist32);
+            drainWide<NS>(queue, qn, hist32);
             qn = 0;
          }
       }
@@ -496,9 +499,9 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    }
    // the queue holds ranks only (no item coordinates): it is drained when full and once here
    if (G::LANEQ) {
-      if (__any_sync(FULL, qa != qLane0)) { drainLanes(queue, (int)((qa - qLane0) >> 8), hist32); }
+      if (__any_sync(FULL, qa != qLane0)) { drainLanes<NS>(queue, (int)((qa - qLane0) >> 8), hist32); }
    } else if (qn > 0) {
-      drainWide(queue, qn, hist32);
+      drainWide<NS>(queue, qn, hist32);
    }
    if (fault) {
       if (lane == 0) { atomicOr(&gTmaFault, 1u); }
@@ -526,7 +529,7 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    if (threadIdx.x == 0) {
       uint32_t n1 = 0, n2 = 0, nr[kTmMaxK + 1];
       for (int r = 0; r <= kTmMaxK; r++) {
-         nr[r] = rowTot[r] - n1 - n2;
+         nr[r] = rowTot[r] - n1 - (NS == 3 ? n2 : 0u);
          n2 = n1;
          n1 = nr[r];
       }
@@ -594,12 +597,12 @@ unsigned thermoTmaFaults(bool clear)
    return v;
 }
 
-template <typename T, bool GE, int CMAX, int V, bool TMA>
-static int launchTmaT(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
+template <typename T, bool GE, int CMAX, int V, bool TMA, int NS>
+static int launchTmaN(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
 {
    using G = TmaGeom<T, V>;
    static std::atomic<int> occ[kTmMaxK + 1];
-   auto kern = thermoTmaBPFD<T, GE, CMAX, V, TMA>;
+   auto kern = thermoTmaBPFD<T, GE, CMAX, V, TMA, NS>;
    const size_t smem = tmaDynBytes<T, V>(a.K);
    const int blocksPerSM = cachedOccupancy(occ[a.K], kern, G::WARPS * 32, smem, tmaDynBytes<T, V>(kTmMaxK));
    long long grid = (a.nItems + G::WARPS - 1) / G::WARPS;
@@ -608,6 +611,26 @@ static int launchTmaT(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
    if (grid < 1) { grid = 1; }
    kern<<<(unsigned)grid, G::WARPS * 32, smem, s>>>(a, tm);
    return cudaFail(cudaGetLastError(), "thermoTmaBPFD launch");
+}
+
+// Whether a cell gets two code slots instead of three. With few thresholds cells rarely cross more
+// than two, and a third slot is one shared atomic and three instructions per row spent on discarded
+// counts; but cells that do cross more are queued, and where there are many of them (a distance field
+// with noise near its surfaces) that costs more. Two / three slots (B200, us): 512^3 FP32 GRF 5
+// thresholds 265 / 286, 8 269 / 287; 256 x 1024 x 1024 FP32 plane waves 8 503 / 536; 512^3 FP64 GRF 6 284 /
+// 304; balls with noise: 256^3 FP32 5 54 / 56, 128^3 6 17.3 / 16.6, 8 22.8 / 18.1, 256 x 256 x 512 FP64 7
+// 89.4 / 89.3, 8 95.6 / 90.3, 400 x 512 x 512 FP32 8 238 / 232.
+static bool twoSlots(const FusedArgs &a, bool f32)
+{
+   const double voxels = (double)a.X * a.Y * a.Z;
+   return a.K <= 5 || (a.K == 6 && voxels >= (double)(1 << 22)) || (a.K <= 8 && f32 && voxels >= (double)(1 << 26));
+}
+
+template <typename T, bool GE, int CMAX, int V, bool TMA>
+static int launchTmaT(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
+{
+   if (V == 0 && twoSlots(a, sizeof(T) == 4)) { return launchTmaN<T, GE, CMAX, V, TMA, V == 0 ? 2 : 3>(a, tm, s); }
+   return launchTmaN<T, GE, CMAX, V, TMA, 3>(a, tm, s);
 }
 
 // Thresholds sharing rank-table buckets (four candidates), and fields without a tensor map, take the

@@ -38,3 +38,18 @@ def test_alignment_does_not_change_counts(mkf, cuda, dtype, shape):
         for m in (4, 6):
             t = np.linspace(-1.3, 1.4, k)
             assert torch.equal(mkf.field_bpfd(aligned, t, m), mkf.field_bpfd(tight, t, m)), (k, m)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("shape", [(60, 190, 352), (130, 190, 352), (256, 512, 512)])
+def test_slot_rule_sizes(mkf, cuda, dtype, shape):
+    """Noise fields (cells crossing any number of the thresholds) at the sizes where a cell gets two or
+    three code slots, 5 to 9 thresholds: the same counts as one threshold at a time."""
+    import torch
+
+    g = torch.Generator(device=cuda).manual_seed(shape[0])
+    f = torch.randn(shape, dtype=getattr(torch, dtype), device=cuda, generator=g)
+    for k, m in ((5, 4), (6, 6), (7, 1), (8, 4), (9, 3)):
+        t = np.linspace(-1.1, 1.2, k)
+        got = mkf.field_bpfd(f, t, m)
+        assert torch.equal(got, torch.cat([mkf.field_bpfd(f, [v], m) for v in t])), (k, m)
