@@ -35,12 +35,10 @@ namespace mkf {
 // One warp counts one work item (31 x positions, TY row pairs, D planes) of the field described
 // by `a` into the CTA's histogram and all-ones totals. Returns the item's number of cells.
 // INNER: the field has X >= 32, Y > TY, and a positive row stride whose TY multiple fits 32 bits
-// in bytes. NSLOT: 3 mixed-code slots, or 1 for one threshold (a cell then has at most one).
-// CMAX: rank-table candidates compared per element (1, or 4 when thresholds share buckets).
-template <typename T, int TY, bool GE, int NSLOT, bool INNER, int CMAX, typename P>
+// in bytes. CMAX: rank-table candidates compared per element (1, or 4 when thresholds share buckets).
+template <typename T, int TY, bool GE, bool INNER, int CMAX, typename P>
 __device__ __forceinline__ unsigned long long warpItem(const P &a, long long it, ThermoShared &S, uint32_t *sHist)
 {
-   static_assert(NSLOT == 1 || NSLOT == 3, "one or three slots");
    constexpr int W = sizeof(T) / 4;  // 32-bit words per element; the ranked word is the last one
    const int lane = threadIdx.x & 31;
    const int K = a.K;
@@ -175,18 +173,14 @@ __device__ __forceinline__ unsigned long long warpItem(const P &a, long long it,
             const uint32_t D0 = R0 + rmin * 0xFEFEFEFFu;         // R0 - rmin per byte (no borrows)
             const uint32_t D1s = R1 * 16u + rmin * 0xEFEFEFF0u;  // (R1 - rmin per byte) << 4
             const uint32_t b0 = gatherBits((D0 & 0x01010101u) | (D1s & 0x10101010u), 0x01020408u);
-            if (NSLOT == 1) {
-               redShared(spread != 0 ? rowAddr + (b0 << 2) : trash);
-            } else {
-               const uint32_t b1 = gatherBits((D0 & 0x02020202u) | (D1s & 0x20202020u), 0x00810204u);
-               const bool fast = spread < 4;
-               redSharedAt<0>(fast && spread > 0 ? (b0 | b1) * 4u + rowAddr : trash);
-               redSharedAt<kHistRow * 4>(fast && spread > 1 ? b1 * 4u + rowAddr : trash);
-               redSharedAt<kHistRow * 8>(fast && spread > 2 ? (b0 & b1) * 4u + rowAddr : trash);
-               if (!fast) {  // counted after the row loop: one copy of that code, not one per row
-                  wq[nwq] = make_uint4(R0, R1, rmin, rmax);
-                  ++nwq;
-               }
+            const uint32_t b1 = gatherBits((D0 & 0x02020202u) | (D1s & 0x20202020u), 0x00810204u);
+            const bool fast = spread < 4;
+            redSharedAt<0>(fast && spread > 0 ? (b0 | b1) * 4u + rowAddr : trash);
+            redSharedAt<kHistRow * 4>(fast && spread > 1 ? b1 * 4u + rowAddr : trash);
+            redSharedAt<kHistRow * 8>(fast && spread > 2 ? (b0 & b1) * 4u + rowAddr : trash);
+            if (!fast) {  // counted after the row loop: one copy of that code, not one per row
+               wq[nwq] = make_uint4(R0, R1, rmin, rmax);
+               ++nwq;
             }
          }
          sF[j] = fc;
@@ -232,7 +226,7 @@ __device__ __forceinline__ unsigned long long warpItem(const P &a, long long it,
    return (unsigned long long)(xe - xs) * (unsigned)(jhi - jlo) * (unsigned)nPln;
 }
 
-template <typename T, int TY, bool GE, int NSLOT, bool INNER, int CMAX>
+template <typename T, int TY, bool GE, bool INNER, int CMAX>
 __global__ void __launch_bounds__(kThWarps * 32, THERMO_MINB) thermoBPFD(const __grid_constant__ FusedArgs a)
 {
    __shared__ ThermoShared S;
@@ -241,7 +235,7 @@ __global__ void __launch_bounds__(kThWarps * 32, THERMO_MINB) thermoBPFD(const _
    const long long gw = (long long)blockIdx.x * kThWarps + (threadIdx.x >> 5);
    const long long nw = (long long)gridDim.x * kThWarps;
    unsigned long long cells = 0;
-   for (long long it = gw; it < a.nItems; it += nw) { cells += warpItem<T, TY, GE, NSLOT, INNER, CMAX>(a, it, S, sHist); }
+   for (long long it = gw; it < a.nItems; it += nw) { cells += warpItem<T, TY, GE, INNER, CMAX>(a, it, S, sHist); }
    if ((threadIdx.x & 31) == 0 && cells) { atomicAdd(&S.cells, cells); }
    ctaFlush(a, S, sHist);
 }
@@ -286,7 +280,7 @@ __global__ void __launch_bounds__(kThWarps * 32, THERMO_MINB) thermoBatch(const 
          cur = ch.field;
       }
       for (long long it = ch.begin + warp; it < ch.end; it += kThWarps) {
-         cells += warpItem<T, TY, (V & 1) != 0, kThSlots, (V & 4) != 0, (V & 8) ? 4 : 1>(F, it, S, sHist);
+         cells += warpItem<T, TY, (V & 1) != 0, (V & 4) != 0, (V & 8) ? 4 : 1>(F, it, S, sHist);
       }
    }
    if (cur >= 0) {
@@ -313,11 +307,11 @@ static uint32_t thresholdKey(double t, int enc, bool ge)
    return sortKey(u);
 }
 
-template <typename T, int TY, bool GE, int NSLOT, bool INNER, int CMAX>
+template <typename T, int TY, bool GE, bool INNER, int CMAX>
 static int launchThermoT(const FusedArgs &a, cudaStream_t s)
 {
    static std::atomic<int> occ[MKF_MAX_THRESH + 1];  // resident CTAs for each K's histogram size
-   auto kern = thermoBPFD<T, TY, GE, NSLOT, INNER, CMAX>;
+   auto kern = thermoBPFD<T, TY, GE, INNER, CMAX>;
    const int blocksPerSM = cachedOccupancy(occ[a.K], kern, kThWarps * 32, thermoDynBytes(a.K), thermoDynBytes(MKF_MAX_THRESH));
    long long grid = (a.nItems + kThWarps - 1) / kThWarps;
    const long long cap = (long long)smCount() * blocksPerSM;
@@ -452,12 +446,10 @@ template <typename T, bool GE>
 static int launchThermoG(const FusedArgs &a, bool inner, cudaStream_t s)
 {
    constexpr int TY = THERMO_TY;
-   // one threshold: a cell has at most one mixed code (and the rank table one candidate)
-   if (a.K == 1) { return inner ? launchThermoT<T, TY, GE, 1, true, 1>(a, s) : launchThermoT<T, TY, GE, 1, false, 1>(a, s); }
    if (a.lutC > 1) {
-      return inner ? launchThermoT<T, TY, GE, kThSlots, true, 4>(a, s) : launchThermoT<T, TY, GE, kThSlots, false, 4>(a, s);
+      return inner ? launchThermoT<T, TY, GE, true, 4>(a, s) : launchThermoT<T, TY, GE, false, 4>(a, s);
    }
-   return inner ? launchThermoT<T, TY, GE, kThSlots, true, 1>(a, s) : launchThermoT<T, TY, GE, kThSlots, false, 1>(a, s);
+   return inner ? launchThermoT<T, TY, GE, true, 1>(a, s) : launchThermoT<T, TY, GE, false, 1>(a, s);
 }
 
 int launchThermo(FusedArgs &a, int enc, cudaStream_t s)

@@ -20,7 +20,6 @@ static constexpr int kThWarps = 8;
 // Untuned fields get at least this many work items per SM (the slab depth is halved until they
 // do): measured on 128^3 to 512^3 fields with 16 thresholds.
 static constexpr int kThItemsPerSM = 14;
-static constexpr int kThSlots = 3;       // unpredicated mixed-code slots per cell (K > 1)
 static constexpr int kThMaxDepth = 255;  // planes per work item the all-ones counters can hold
 static constexpr int kLutShift = 18;
 static constexpr int kLutSize = 1 << (32 - kLutShift);
