@@ -452,6 +452,30 @@ static int launchThermoG(const FusedArgs &a, bool inner, cudaStream_t s)
    return inner ? launchThermoT<T, TY, GE, true, 1>(a, s) : launchThermoT<T, TY, GE, false, 1>(a, s);
 }
 
+// Slab depth of the staged kernel: the busiest warp's planes (rounds of items of D + 1 planes, one of
+// them the halo, and about half a plane's time to start each) over every number of rounds up to
+// kRounds, with the shallowest slabs that fit; larger fields take the full depth. Against halving the
+// depth until every warp has four items, which left the last round of a field of middle size
+// half empty (B200, us): 384^3 FP32 8 thresholds 149 -> 133, 450 x 390 x 260 FP64 16 154 -> 138, 256^3 FP64 16
+// 68.5 -> 63.2, 333 x 401 x 487 FP64 12 197 -> 190, 512^3 269 -> 266 (FP32, 8), 342 -> 341 (FP64, 16).
+static int ringDepth(long long perPlane, int cellsZ, long long warps)
+{
+   constexpr int kRounds = 32;
+   double best = 0.0;
+   int depth = THERMO_D;
+   for (int r = 1; r <= kRounds; r++) {
+      const long long slabs = std::min<long long>(cellsZ, r * warps / perPlane);
+      if (slabs < 1) { continue; }
+      const int d = (int)((cellsZ + slabs - 1) / slabs);
+      const double cost = r * (d + 1.5);
+      if (d <= THERMO_D && (best == 0.0 || cost < best)) {
+         best = cost;
+         depth = d;
+      }
+   }
+   return depth;
+}
+
 int launchThermo(FusedArgs &a, int enc, cudaStream_t s)
 {
    a.lutC = prepareKeys(a, enc);
@@ -459,8 +483,7 @@ int launchThermo(FusedArgs &a, int enc, cudaStream_t s)
    const long long perPlane = (long long)((a.X - 1 + 30) / 31) * ((a.Y - 1 + THERMO_TY - 1) / THERMO_TY);
    // up to 16 thresholds on fields of at least one tile: tiles staged in shared memory
    if (thermoRingEligible(a)) {
-      itemGrid(a, tunedDepth(kFamThermoTma, enc, a.K, a.X, a.Y, a.Z,
-                             sizeDepth(THERMO_D, perPlane, a.Z, (long long)smCount() * kTmItemsPerSM)));
+      itemGrid(a, tunedDepth(kFamThermoTma, enc, a.K, a.X, a.Y, a.Z, ringDepth(perPlane, a.Z - 1, (long long)smCount() * kTmWarpsPerSM)));
       const int rc = launchThermoRing(a, enc, tunedVariant(kFamThermoTma, enc, a.K, a.X, a.Y, a.Z, 0), s);
       if (rc != MKF_ERR_UNSUPPORTED) { return rc; }
    }

@@ -327,7 +327,7 @@ __device__ __forceinline__ uint32_t cellCode(uint32_t R0, uint32_t R1, uint32_t 
 
 // The rank-table kernel with its tiles staged in shared memory (thermo_tma.cu): whether it takes this
 // pass (after prepareKeys), and its launch (after itemGrid; MKF_ERR_UNSUPPORTED when it does not).
-static constexpr int kTmItemsPerSM = 80;  // four items per resident warp (20 per SM)
+static constexpr int kTmWarpsPerSM = 20;  // resident warps of the default variant
 bool thermoRingEligible(const FusedArgs &a);
 // variant: CTA shape, histogram privatisation and queue kind (kTmVariants in thermo_tma.cu,
 // kTmNumVariants of them), 0 = default; fields off 16-byte boundaries have the default only.
