@@ -109,8 +109,8 @@ int mkfFieldBPFDHostNoAlloc(uint64_t *pBPFDH, const MKFFieldDesc *pF, const MKFT
 /* ---- many fields, one launch (no original counterpart; the original runs one field per call) ---- */
 /* Fields i = 0..nF-1 (device pointers, any shapes, FP32/FP64) with threshold sets pT[i]; the counts
  * of field i are rows nT_0 + ... + nT_{i-1} onwards of pBPFD (device, overwritten). One persistent
- * launch walks a work list of (field, item chunk) entries; fields whose thresholds mix relations
- * are counted by their own pass. A plan keeps the work list on the device so the same batch (same
+ * launch walks a work list of (field, item chunk) entries; fields large enough to fill the GPU
+ * on their own are counted by their own pass. A plan keeps the work list on the device so the same batch (same
  * buffers, new contents) can be launched again, also inside a CUDA graph. */
 typedef struct MKFBatchPlan MKFBatchPlan;
 /* Unless mkfSetTuning(0) switched it off, creation times one launch of the batch for each candidate

@@ -85,7 +85,6 @@ static int wordThresholds(const FusedArgs &a, int enc)
    return enc == ENC_F64 && large && !tmaRowsAligned(a, enc) ? 5 : 4;
 }
 
-
 void fillRankArgs(FusedArgs &a, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, int row0)
 {
    memset(&a, 0, sizeof(a));

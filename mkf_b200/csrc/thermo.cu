@@ -1,4 +1,6 @@
-// thermo.cu - fused counting kernel for threshold sets that share one relation (< <= > >=).
+// thermo.cu - fused counting kernel for threshold sets that share one relation (< <= > >=), reading
+// the field straight from global memory: 17 to 32 thresholds, fields too small for the staged
+// kernel's tiles (thermo_tma.cu), and the small fields of a batch with more than kWordMaxK thresholds.
 //
 // Sorted thresholds make an element's K map bits a thermometer, bits[k] = (k < rank), so an
 // element reduces to one rank 0..K. The rank is found with a table over order-preserving 32-bit
@@ -20,8 +22,7 @@
 // packed ranks only for k in between: three unpredicated atomic slots cover the cells spanning up
 // to 3 thresholds (99 % on a smooth field); wider cells are queued and counted after the row loop.
 // Codes go to the per-CTA [K][256] shared histogram. All-ones counts are summed per threshold with
-// bit-sliced carry-save adders and all-zeros counts follow from the number of cells, as in
-// fused.cu. The kernel is bound by the integer ALU pipe, so arithmetic that can be a multiply-add
+// bit-sliced carry-save adders and all-zeros counts follow from the number of cells. The kernel is bound by the integer ALU pipe, so arithmetic that can be a multiply-add
 // is written as one (it runs on the FMA pipe).
 #include <algorithm>
 #include <cmath>
@@ -330,8 +331,7 @@ static bool innerTiles(const P &a, int enc)
 }
 
 // Fill the key table of a thermometer pass and return the most thresholds sharing one bucket of
-// the rank table (1..4), or 0 when more share one (such passes use the binary-search kernel of
-// fused.cu).
+// the rank table (1..4), or 0 when more share one (the word kernels count such passes).
 template <typename P>
 static int prepareKeys(P &a, int enc)
 {

@@ -1,5 +1,5 @@
 // thermo_tma.cu - the rank-table counting kernel with plane tiles staged in shared memory (by TMA on
-// fields whose rows start on 16-byte boundaries, else by cp.async), for 3..16 thresholds of one relation
+// fields whose rows start on 16-byte boundaries, else by cp.async), for 5..16 thresholds of one relation
 // (< <= > >=).
 //
 // The method is thermo.cu's (sorted thresholds: an element's K map bits are a thermometer, found
@@ -44,7 +44,7 @@ namespace mkf {
 // Kernel variants (the CTA shape, the histogram privatisation and the wide-cell queue mkfTune
 // chooses among; 0 is the default): warps per CTA (one CTA per SM), ring stages for FP64 / FP32
 // tiles, histogram copies (lane parity picks the copy; one copy halves that shared memory), queue
-// kind for the cells crossing four or more thresholds (1: one queue per lane, appended without a
+// kind for the cells crossing more thresholds than slots (1: one queue per lane, appended without a
 // warp vote and drained by the whole warp; 0: one queue per warp, appended through a ballot).
 // Measured on 512^3 Gaussian fields: the per-lane queue is 4-16 % faster for 5-12 thresholds and
 // even at 16 (where more cells are wide); 16 warps with 3 stages need the warp queue's smaller
