@@ -82,6 +82,9 @@ struct TmaGeom
    static constexpr int QWORDS = LANEQ ? kTmLaneQ * 32 : kTmQueue + 1;  // queue entries per warp
 };
 
+// How a ring stage is filled (the kernel's COPY).
+enum { kCopyElems, kCopyTma, kCopyBlocks };
+
 // Set when a wait of this kernel ran out of polls (never in a correct run); read by mkfKernelFaults.
 __device__ unsigned gTmaFault;
 
@@ -247,16 +250,24 @@ __device__ __forceinline__ TmItem itemOf(const FusedArgs &a, long long it, int l
    return m;
 }
 
-// TMA false: fields that a tensor map cannot take (rows off 16-byte boundaries, strided x). Every lane
-// then copies its own column of the tile with cp.async, one element per row, into the same ring, and
-// waits for its own copies only; the rest is the same. Against thermo.cu, which took these fields
+// COPY: how the ring is filled. Fields that a tensor map cannot take use cp.async: with strided x every
+// lane copies its own column of the tile, one element per row, and waits for its own copies only; where
+// only the alignment of the rows is off, the warp copies the 16-byte blocks that the rows touch, and a
+// row is read from where it starts in its first block. The rest is the same. Against thermo.cu, which took these fields
 // before (B200, us): 333 x 401 x 487 FP64, 12 thresholds 240 -> 197, 16 265 -> 212; 301 x 333 x 277 FP32, 8
-// 110 -> 77; 100 x 101 x 99 FP64, 12 27 -> 18.
-template <typename T, bool GE, int CMAX, int V, bool TMA, int NS>
+// 110 -> 77; 100 x 101 x 99 FP64, 12 27 -> 18. Blocks instead of elements (5 or 3 copies per lane and plane
+// instead of 9, and half the requests to L2): 333 x 401 x 487 FP64, 12 196 -> 158, 16 212 -> 178, plane
+// waves, 6 186 -> 145; 301 x 333 x 277 FP64, 12 90 -> 77; 401 x 403 x 405 FP32, 8 176 -> 156.
+template <typename T, bool GE, int CMAX, int V, int COPY, int NS>
 __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
     thermoTmaBPFD(const __grid_constant__ FusedArgs a, const __grid_constant__ CUtensorMap tm)
 {
    using G = TmaGeom<T, V>;
+   constexpr bool TMA = COPY == kCopyTma;
+   constexpr int B = (int)sizeof(T), ROWB = G::BX * B;  // bytes of an element, of a tile row
+   constexpr int NB = 2 * B;                            // blocks of a row of 32 elements
+   constexpr int NR = 32 / NB;                          // rows per copy of blocks
+   static_assert(ROWB == 16 * (NB + 1) && 8 % NR == 0 && NB + kTmRows <= 32, "rows of NB + 1 blocks");
    constexpr int kTmWarps = G::WARPS, kHistCopies = G::COPIES;
    constexpr int W = sizeof(T) / 4;   // 32-bit words per element; the ranked word is the last
    constexpr int S = G::STAGES;
@@ -299,13 +310,19 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    // producer cursor (every lane tracks it; lane 0 issues): item, plane, tile coordinates
    long long pIt = first;
    int pP = 0, pX = 0, pY = 0, pZ = 0, pN = -1;
-   const char *pCol = nullptr;  // (not TMA) this lane's element of the tile's first row
+   // (elements) this lane's element of the tile's first row; (blocks) this lane's block of its row among
+   // the first NR, plus the row's offset in a block
+   const char *pCol = nullptr;
    auto begin = [&]() {
       if (pIt < a.nItems) {
          const TmItem m = itemOf<G::ALIGN>(a, pIt, lane);
          pX = m.xa; pY = m.y0; pZ = m.z0; pN = m.nPln;
-         if (!TMA) {
-            pCol = (const char *)a.f + ((int64_t)(m.xa + m.xoff + lane) * a.sx + (int64_t)m.y0 * a.sy + (int64_t)m.z0 * a.sz) * (int64_t)sizeof(T);
+         if (COPY == kCopyElems) {
+            pCol = (const char *)a.f + ((int64_t)(m.xa + m.xoff + lane) * a.sx + (int64_t)m.y0 * a.sy + (int64_t)m.z0 * a.sz) * (int64_t)B;
+         }
+         if (COPY == kCopyBlocks) {
+            pCol = (const char *)a.f + ((int64_t)(m.xa + m.xoff) + (int64_t)(m.y0 + lane / NB) * a.sy + (int64_t)m.z0 * a.sz) * (int64_t)B +
+                   16 * (lane % NB);
          }
       }
    };
@@ -316,15 +333,32 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
          const uint32_t st = gp % S;
          if (TMA) {
             if (lane == 0) { tmaTile3D(&tm, ringW + st * G::PITCH, bar0 + 8u * st, pX, pY, pZ + pP, G::BYTES); }
-         } else {
-            const uint32_t dst = ringW + st * G::PITCH + (uint32_t)(lane * (int)sizeof(T));
+         } else if (COPY == kCopyElems) {
+            const uint32_t dst = ringW + st * G::PITCH + (uint32_t)(lane * B);
             const char *q = pCol;
 #pragma unroll
             for (int j = 0; j < kTmRows; ++j) {
-               asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + (uint32_t)(j * G::BX * (int)sizeof(T))), "l"(q), "n"((int)sizeof(T)) : "memory");
-               q += a.sy * (int64_t)sizeof(T);
+               asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + (uint32_t)(j * ROWB)), "l"(q), "n"(B) : "memory");
+               q += a.sy * (int64_t)B;
             }
-            pCol += a.sz * (int64_t)sizeof(T);
+            pCol += a.sz * (int64_t)B;
+         } else {
+            // NB blocks of NR rows at a time; then the ninth row's and, by the next nine lanes, each row's
+            // last block, which it touches only where it does not start on a boundary. Every block copied
+            // holds a byte of the field, so it lies in the field's allocation.
+            const uint32_t tile = ringW + st * G::PITCH, dst = tile + (uint32_t)((lane / NB) * ROWB + (lane % NB) * 16);
+            const char *q = pCol;
+#pragma unroll
+            for (int k = 0; k < 8 / NR; ++k) {
+               asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(k * NR * ROWB)), "l"((uintptr_t)q & ~(uintptr_t)15) : "memory");
+               q += a.sy * (int64_t)(NR * B);
+            }
+            const int row = lane < NB ? 8 : lane - NB, blk = lane < NB ? lane : NB;
+            q = pCol + a.sy * (int64_t)((row - lane / NB) * B) + 16 * (blk - lane % NB);
+            if (lane < NB || (lane < NB + kTmRows && ((uintptr_t)q & 15) != 0)) {
+               asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tile + (uint32_t)(row * ROWB + blk * 16)), "l"((uintptr_t)q & ~(uintptr_t)15) : "memory");
+            }
+            pCol += a.sz * (int64_t)B;
          }
          ++gp;
          if (++pP > pN) {
@@ -339,6 +373,7 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
 
    uint32_t g = 0;  // planes consumed by this warp
    bool fault = false;
+   uint32_t rowLo = 0;  // (blocks) low address bits of the first row of plane g's tile
    // wait for plane g's tile, rank the lane's column (9 rows), refill the stage of plane g - 1
    auto plane = [&](int xoff, uint32_t (&r)[kTmRows]) -> bool {
       const uint32_t st = g % S;
@@ -347,10 +382,19 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
          if (!__all_sync(FULL, mbarWait(bar0 + 8u * st, (g / S) & 1u))) { return false; }
       } else {
          asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+         if (COPY == kCopyBlocks) { __syncwarp(); }  // (the other lanes' copies too)
       }
       // this lane's column of the plane tile (the mbarrier wait orders these loads after the copy)
-      const T *col = reinterpret_cast<const T *>(ring + (size_t)(warp * S + (int)st) * G::PITCH) + (TMA ? xoff : 0) + lane;
-      const uint32_t *colW = reinterpret_cast<const uint32_t *>(col) + (W - 1);
+      // (blocks: a row starts rowLo's offset into its first block; the offsets repeat every NO rows)
+      constexpr int NO = COPY == kCopyBlocks ? 16 / B : 1;
+      const unsigned char *tile = ring + (size_t)(warp * S + (int)st) * G::PITCH;
+      const T *col[NO];
+#pragma unroll
+      for (int o = 0; o < NO; ++o) {
+         const uint32_t sh = COPY == kCopyBlocks ? (rowLo + (uint32_t)(o * B) * (uint32_t)a.sy) & 15u : 0u;
+         col[o] = reinterpret_cast<const T *>(tile + sh) + (TMA ? xoff : 0) + lane;
+      }
+      if (COPY == kCopyBlocks) { rowLo += (uint32_t)a.sz * (uint32_t)B; }
       bool slow = false;   // a FP64 high word equal to a threshold's
       uint32_t rOr = 0;    // slow-path buckets rank above 32
       // The table finds the rank of the element's bucket from its top bits, a comparison with the
@@ -360,7 +404,8 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
       // 16 thresholds, and whole elements 4 % (8-byte candidates): there the shared-memory pipe decides.
 #pragma unroll
       for (int j = 0; j < kTmRows; ++j) {
-         const uint32_t top = W == 1 ? colW[j * G::BX * W] : sortKey(colW[j * G::BX * W]);
+         const uint32_t word = reinterpret_cast<const uint32_t *>(col[j % NO] + j * G::BX)[W - 1];
+         const uint32_t top = W == 1 ? word : sortKey(word);
          const uint32_t r0 = Sh.lut[top >> kLutShift];
          uint32_t rr = r0;
 #pragma unroll
@@ -382,7 +427,7 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
       if (__any_sync(FULL, slow)) {
          if (slow) {
 #pragma unroll
-            for (int j = 0; j < kTmRows; ++j) { r[j] = exactRankAt<T, GE>(col + j * G::BX, Sh.tlo, Sh.thi, K, nanRank); }
+            for (int j = 0; j < kTmRows; ++j) { r[j] = exactRankAt<T, GE>(col[j % NO] + j * G::BX, Sh.tlo, Sh.thi, K, nanRank); }
          }
       }
       __syncwarp();
@@ -409,6 +454,9 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    uint32_t qa = qLane0;
    for (long long it = first; it < a.nItems; it += nw) {
       const TmItem m = itemOf<G::ALIGN>(a, it, lane);
+      if (COPY == kCopyBlocks) {
+         rowLo = (uint32_t)(uintptr_t)a.f + ((uint32_t)(m.xa + m.xoff) + (uint32_t)m.y0 * (uint32_t)a.sy + (uint32_t)m.z0 * (uint32_t)a.sz) * (uint32_t)B;
+      }
       cells += m.cells;
       masked += (8u - (uint32_t)__popc(m.rowsOK)) * (uint32_t)m.nPln;
       uint32_t sF[8], sV[8];  // previous plane: face ranks (bytes), minimum of the face pairs
@@ -597,12 +645,12 @@ unsigned thermoTmaFaults(bool clear)
    return v;
 }
 
-template <typename T, bool GE, int CMAX, int V, bool TMA, int NS>
+template <typename T, bool GE, int CMAX, int V, int COPY, int NS>
 static int launchTmaN(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
 {
    using G = TmaGeom<T, V>;
    static std::atomic<int> occ[kTmMaxK + 1];
-   auto kern = thermoTmaBPFD<T, GE, CMAX, V, TMA, NS>;
+   auto kern = thermoTmaBPFD<T, GE, CMAX, V, COPY, NS>;
    const size_t smem = tmaDynBytes<T, V>(a.K);
    const int blocksPerSM = cachedOccupancy(occ[a.K], kern, G::WARPS * 32, smem, tmaDynBytes<T, V>(kTmMaxK));
    long long grid = (a.nItems + G::WARPS - 1) / G::WARPS;
@@ -626,11 +674,11 @@ static bool twoSlots(const FusedArgs &a, bool f32)
    return a.K <= 5 || (a.K == 6 && voxels >= (double)(1 << 22)) || (a.K <= 8 && f32 && voxels >= (double)(1 << 26));
 }
 
-template <typename T, bool GE, int CMAX, int V, bool TMA>
+template <typename T, bool GE, int CMAX, int V, int COPY>
 static int launchTmaT(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
 {
-   if (V == 0 && twoSlots(a, sizeof(T) == 4)) { return launchTmaN<T, GE, CMAX, V, TMA, V == 0 ? 2 : 3>(a, tm, s); }
-   return launchTmaN<T, GE, CMAX, V, TMA, 3>(a, tm, s);
+   if (V == 0 && twoSlots(a, sizeof(T) == 4)) { return launchTmaN<T, GE, CMAX, V, COPY, V == 0 ? 2 : 3>(a, tm, s); }
+   return launchTmaN<T, GE, CMAX, V, COPY, 3>(a, tm, s);
 }
 
 // Thresholds sharing rank-table buckets (four candidates), and fields without a tensor map, take the
@@ -638,13 +686,14 @@ static int launchTmaT(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
 template <typename T, bool GE>
 static int launchTmaG(const FusedArgs &a, const CUtensorMap &tm, bool tma, int variant, cudaStream_t s)
 {
-   if (!tma) { return a.lutC > 1 ? launchTmaT<T, GE, 4, 0, false>(a, tm, s) : launchTmaT<T, GE, 1, 0, false>(a, tm, s); }
-   if (a.lutC > 1) { return launchTmaT<T, GE, 4, 0, true>(a, tm, s); }
+   if (!tma && a.sx == 1) { return a.lutC > 1 ? launchTmaT<T, GE, 4, 0, kCopyBlocks>(a, tm, s) : launchTmaT<T, GE, 1, 0, kCopyBlocks>(a, tm, s); }
+   if (!tma) { return a.lutC > 1 ? launchTmaT<T, GE, 4, 0, kCopyElems>(a, tm, s) : launchTmaT<T, GE, 1, 0, kCopyElems>(a, tm, s); }
+   if (a.lutC > 1) { return launchTmaT<T, GE, 4, 0, kCopyTma>(a, tm, s); }
    switch (variant) {
-      case 1: return launchTmaT<T, GE, 1, 1, true>(a, tm, s);
-      case 2: return launchTmaT<T, GE, 1, 2, true>(a, tm, s);
-      case 3: return launchTmaT<T, GE, 1, 3, true>(a, tm, s);
-      default: return launchTmaT<T, GE, 1, 0, true>(a, tm, s);
+      case 1: return launchTmaT<T, GE, 1, 1, kCopyTma>(a, tm, s);
+      case 2: return launchTmaT<T, GE, 1, 2, kCopyTma>(a, tm, s);
+      case 3: return launchTmaT<T, GE, 1, 3, kCopyTma>(a, tm, s);
+      default: return launchTmaT<T, GE, 1, 0, kCopyTma>(a, tm, s);
    }
 }
 
