@@ -1,5 +1,5 @@
 // ballot.cu - fused counting kernel for one threshold on fields of middle size, and for a few of
-// one test on larger FP64 fields: map words packed by warp votes from registers.
+// one test on larger FP64 fields and the largest FP32 fields off 16-byte boundaries: map words packed by warp votes from registers.
 //
 // The other kernel for few thresholds (words.cuh) lets each lane pack its own row from a copy of the
 // tile in shared memory. That costs fewer instructions per threshold, but a FP64 tile row holds only
@@ -233,6 +233,13 @@ static int launchBallotM(const WordTask &a, int enc, cudaStream_t s)
       if (a.K == 4) { return launchBallotT<T, MODE, 4, true, 2, false>(a, s); }
       if (a.K == 5) { return launchBallotT<T, MODE, 5, true, 2, false>(a, s); }
    }
+   if constexpr (F32 && MODE < 3) {
+      if (a.K == 2 && a.D >= kBlPfDepth) { return launchBallotT<T, MODE, 2, true, 2, true>(a, s); }
+      if (a.K == 2) { return launchBallotT<T, MODE, 2, true, 4, false>(a, s); }
+      if (a.K == 3) { return launchBallotT<T, MODE, 3, true, 3, false>(a, s); }
+      if (a.K == 4) { return launchBallotT<T, MODE, 4, true, 3, false>(a, s); }
+      if (a.K == 5) { return launchBallotT<T, MODE, 5, true, 3, false>(a, s); }
+   }
    if (!innerTiles(a, enc)) { return launchBallotT<T, MODE, 1, false, 2, false>(a, s); }
    if (F32 && a.D >= kBlPfDepth) { return launchBallotT<T, MODE, 1, true, 2, F32>(a, s); }
    return launchBallotT<T, MODE, 1, true, F32 ? 4 : 2, false>(a, s);
@@ -253,15 +260,22 @@ static int dispatchBallot(const WordTask &a, int enc, cudaStream_t s)
 // 128 x 2048 x 2048 398 / 359; FP64 64^3 8.0 / 6.1, 128^3 9.2 / 9.6, 256 x 512 x 512 86 / 97,
 // 333 x 401 x 487 85 / 111. Four thresholds on larger FP64 fields: 256 x 512 x 512 plane waves 131 / 146,
 // GRF 158 / 161. Two to five on FP64 rows off 16-byte boundaries, where the other kernel's tile rows are
-// a ninth wider and fewer warps fit: 333 x 401 x 487 GRF, 3 thresholds 155 / 170, 4 158 / 181, plane
-// waves, 5 (against the rank table) 163 / 190; 301 x 333 x 277, 2 61 / 64, 3 82 / 79, 4 85 / 87;
-// 100 x 101 x 99, 3 18 / 12.
+// a ninth wider and fewer warps fit: 333 x 401 x 487 GRF, 3 thresholds 155 / 170, 4 158 / 181;
+// 301 x 333 x 277, 2 61 / 64, 3 82 / 79, 4 85 / 87; 100 x 101 x 99, 3 18 / 12.
+// The largest FP32 fields off 16-byte boundaries: this kernel gains where most tiles are uniform, and
+// the others' cost does not depend on the content (5: the rank table), 599 x 611 x 515, balls with noise: 2
+// thresholds 202 / 213, 3 241 / 293, 4 292 / 371, 5 347 / 387; plane waves 258 / 220, 340 / 311, 320 / 385, 402 /
+// 388; GRF 310 / 269, 427 / 378, 426 / 425, 527 / 391; 861 x 841 x 512 balls, 5 533 / 725; 478 x 768 x 993
+// GRF, 1 316 / 332. At 499 x 501 x 503 (below the line) balls 156 / 149, 185 / 193, 223 / 220, 269 / 268, GRF
+// 221 / 186, 319 / 257, 315 / 249, 381 / 271. The content is not known here; the line keeps the balls' worst
+// case.
 bool useBallots(const WordTask &a, int enc)
 {
    const double voxels = (double)a.X * a.Y * a.Z;
-   if (a.K == 1) { return voxels >= (double)(1 << 20) && (enc == ENC_F64 || voxels < (double)(1 << 26)); }
-   if (enc != ENC_F64 || a.K > 5 || voxels < (double)(1 << 24) || !innerTiles(a, enc)) { return false; }
-   if (a.K != 4 && wordRowsAligned(a, enc)) { return false; }
+   const bool largeF32 = enc == ENC_F32 && voxels >= (double)(1 << 27) && !wordRowsAligned(a, enc);
+   if (a.K == 1) { return voxels >= (double)(1 << 20) && (enc == ENC_F64 || voxels < (double)(1 << 26) || largeF32); }
+   if (!(enc == ENC_F64 || largeF32) || a.K > 5 || voxels < (double)(1 << 24) || !innerTiles(a, enc)) { return false; }
+   if (enc == ENC_F64 && a.K != 4 && wordRowsAligned(a, enc)) { return false; }
    for (int k = 0; k < a.K; k++) {
       if (a.mode[k] != a.mode[0] || a.mode[k] == 3) { return false; }
    }

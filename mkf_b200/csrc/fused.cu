@@ -76,14 +76,10 @@ void splitThresholds(const MKFThreshSet *pT, ThreshSplit &q)
 // Thresholds of one relation that the word kernels count rather than a rank-table kernel, whose cost
 // hardly grows with their number (B200, us, word kernel / rank table): 512^3 FP32 GRF 4 thresholds
 // 244 / 302, 5 325 / 304; 128 x 2048 x 2048 FP32 plane waves 4 739 / 734, 5 947 / 1145; 256 x 512 x 512
-// FP64 GRF 4 158 / 165, 5 221 / 166; rows off 16-byte boundaries: 301 x 333 x 277 FP32 4 72 / 76, 5 83 / 76,
-// 6 95 / 76; 333 x 401 x 487 FP64 4 158 / 192, 5 192 / 193, plane waves 163 / 190;
-// 301 x 333 x 277 FP64 5 104 / 88.
-static int wordThresholds(const FusedArgs &a, int enc)
-{
-   const bool large = (double)a.X * a.Y * a.Z >= (double)(1 << 25);
-   return enc == ENC_F64 && large && !tmaRowsAligned(a, enc) ? 5 : 4;
-}
+// FP64 GRF 4 158 / 165, 5 221 / 166; rows off 16-byte boundaries: 401 x 403 x 405 FP32 GRF 3 130 / 144,
+// 4 150 / 143, plane waves 4 137 / 143; 333 x 401 x 487 FP64 GRF 4 161 / 144, 5 193 / 144, plane waves
+// 4 138 / 144, 5 165 / 145; 100 x 101 x 99 FP64 4 12.2 / 13.0.
+static constexpr int kWordThresholds = 4;
 
 void fillRankArgs(FusedArgs &a, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, int row0)
 {
@@ -175,14 +171,18 @@ int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, Fie
 
 int countVarying(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, cudaStream_t s)
 {
-   if (q.cls >= 0 && q.n > 4) {
+   bool votes = false;  // five thresholds of a large FP32 field off 16-byte boundaries (useBallots)
+   if (q.cls >= 0 && q.n == 5 && pF->enc == ENC_F32) {
+      WordTask w;
+      fillWordTask(w, pF, pT, q, 0, q.n, 0);
+      votes = useBallots(w, pF->enc);
+   }
+   if (q.cls >= 0 && q.n > kWordThresholds && !votes) {
       FusedArgs a;
       fillRankArgs(a, pF, pT, q, 0);
       a.out = out;
-      if (q.n > wordThresholds(a, pF->enc)) {
-         const int rc = launchThermo(a, pF->enc, s);
-         if (rc != MKF_ERR_UNSUPPORTED) { return rc; }
-      }
+      const int rc = launchThermo(a, pF->enc, s);
+      if (rc != MKF_ERR_UNSUPPORTED) { return rc; }
    }
    const int passes = (q.n + kWordMaxK - 1) / kWordMaxK;
    for (int p = 0; p < passes; p++) {

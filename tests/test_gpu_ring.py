@@ -53,3 +53,20 @@ def test_slot_rule_sizes(mkf, cuda, dtype, shape):
         t = np.linspace(-1.1, 1.2, k)
         got = mkf.field_bpfd(f, t, m)
         assert torch.equal(got, torch.cat([mkf.field_bpfd(f, [v], m) for v in t])), (k, m)
+
+
+@pytest.mark.parametrize("shape", [(128, 1023, 1023), (130, 1025, 1023)])
+def test_large_fp32_fields_off_boundaries(mkf, cuda, shape):
+    """Two to five thresholds of one relation below and above 2^27 voxels: the same counts as on aligned
+    rows, and as one threshold at a time."""
+    import torch
+
+    Z, Y, X = shape
+    g = torch.Generator(device=cuda).manual_seed(Z)
+    buf = torch.randn((Z, Y, X + 1), device=cuda, generator=g)
+    aligned, tight = buf[:, :, :X], buf[:, :, :X].contiguous()
+    for k, m in ((1, 5), (2, 4), (3, 6), (4, 1), (5, 3), (5, 4)):
+        t = np.linspace(-1.3, 1.4, k)
+        got = mkf.field_bpfd(tight, t, m)
+        assert torch.equal(got, mkf.field_bpfd(aligned, t, m)), (k, m)
+        assert torch.equal(got, torch.cat([mkf.field_bpfd(tight, [v], m) for v in t])), (k, m)
