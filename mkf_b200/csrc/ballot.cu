@@ -1,5 +1,6 @@
 // ballot.cu - fused counting kernel for one threshold on fields of middle size, and for a few of
-// one test on larger FP64 fields and the largest FP32 fields off 16-byte boundaries: map words packed by warp votes from registers.
+// one test on larger FP64 fields and the largest FP32 fields off 16-byte boundaries: map words packed
+// by warp votes from registers.
 //
 // The other kernel for few thresholds (words.cuh) lets each lane pack its own row from a copy of the
 // tile in shared memory. That costs fewer instructions per threshold, but a FP64 tile row holds only
