@@ -17,33 +17,27 @@ void setError(const char *fmt, ...);
 int cudaFail(cudaError_t e, const char *what);
 int smCount();
 
-// Resident CTAs per SM of `kern` for a block size and dynamic shared-memory size, computed on the
-// first call for a cache slot and kept there (a relaxed atomic: host threads that race compute the
-// same value). maxSmem > 48 KB is first allowed with cudaFuncSetAttribute.
+// Allow `kern` maxSmem bytes of dynamic shared memory on the current device; called before every launch
+// that needs more than 48 KB. The limit belongs to the kernel on one device and goes with a reset of that
+// device, so nothing here remembers that it was set (0.13 us a call).
 template <typename K>
-int cachedOccupancy(std::atomic<int> &slot, K kern, int threads, size_t smem, size_t maxSmem = 0)
+void allowSmem(K kern, size_t maxSmem)
+{
+   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)maxSmem);
+}
+// Resident CTAs per SM of `kern` for a block size and dynamic shared-memory size (allowSmem beforehand
+// above 48 KB), computed on the first call for a cache slot and kept there (a relaxed atomic: host
+// threads that race compute the same value).
+template <typename K>
+int cachedOccupancy(std::atomic<int> &slot, K kern, int threads, size_t smem)
 {
    int v = slot.load(std::memory_order_relaxed);
    if (v > 0) { return v; }
-   if (maxSmem > 48 * 1024) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)maxSmem); }
    int n = 0;
    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem);
    v = n > 0 ? n : 1;
    slot.store(v, std::memory_order_relaxed);
    return v;
-}
-// Allow `kern` maxSmem bytes of dynamic shared memory on the current device (once per device: `done`
-// has a bit for each).
-template <typename K>
-void allowSmem(std::atomic<uint64_t> &done, K kern, size_t maxSmem)
-{
-   int dev = 0;
-   if (cudaGetDevice(&dev) != cudaSuccess) { return; }
-   const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
-   if (done.load(std::memory_order_relaxed) & bit) { return; }
-   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)maxSmem) == cudaSuccess) {
-      done.fetch_or(bit, std::memory_order_relaxed);
-   }
 }
 // Log a message on stderr the way the original library reports CUDA failures (ctuErr).
 void logError(const char *fmt, ...);

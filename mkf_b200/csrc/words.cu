@@ -113,9 +113,8 @@ static void wordGrid(const WordTask &a, int enc, bool mis, int ctas, int &depth,
 template <typename T, bool MOM, int KT, bool MIS>
 static int launchWordsT(WordTask &a, int enc, cudaStream_t s)
 {
-   static std::atomic<uint64_t> allowed{0};
    auto kern = wordBPFD<T, MOM, KT, MIS>;
-   allowSmem(allowed, kern, kWdDynBytes);
+   allowSmem(kern, kWdDynBytes);
    int depth, strip;
    wordGrid(a, enc, MIS, smCount(), depth, strip);
    if (!MOM) { depth = tunedDepth(kFamWords, enc, a.K, a.X, a.Y, a.Z, depth); }

@@ -61,9 +61,8 @@ std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks)
 template <typename T>
 static int launchBatchT(const WordBatchArgs &b, cudaStream_t s)
 {
-   static std::atomic<uint64_t> allowed{0};
    auto kern = wordBatch<T>;
-   allowSmem(allowed, kern, kWdDynBytes);
+   allowSmem(kern, kWdDynBytes);
    long long grid = smCount();
    if (grid > b.nChunks) { grid = b.nChunks; }
    if (grid < 1) { grid = 1; }
