@@ -6,6 +6,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include "mkf_common.cuh"
 #include "binMapUtil.h"
 #include "mkfUtil.h"
@@ -47,6 +49,22 @@ int smCount()
       n = 148;
    }
    return n;
+}
+
+unsigned long long contextId()
+{
+   static const PFN_cuCtxGetId_v12000 fn = [] {
+      void *p = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+          q != cudaDriverEntryPointSuccess) {
+         cudaGetLastError();
+         p = nullptr;
+      }
+      return reinterpret_cast<PFN_cuCtxGetId_v12000>(p);
+   }();
+   unsigned long long id = 0;
+   return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 // Symmetry group of each 2x2x2 pattern under the 48 symmetries of the cube, numbered as the

@@ -17,13 +17,27 @@ void setError(const char *fmt, ...);
 int cudaFail(cudaError_t e, const char *what);
 int smCount();
 
-// Allow `kern` maxSmem bytes of dynamic shared memory on the current device; called before every launch
-// that needs more than 48 KB. The limit belongs to the kernel on one device and goes with a reset of that
-// device, so nothing here remembers that it was set (0.13 us a call).
-template <typename K>
-void allowSmem(K kern, size_t maxSmem)
+// Number of the calling thread's current CUDA context (no two contexts of a process share one, and a
+// device has a new one after a reset); 0 when it is not known. What belongs to a context is kept by this.
+unsigned long long contextId();
+
+// Contexts in which a kernel's shared-memory limit was raised.
+struct SmemAllowed
 {
-   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)maxSmem);
+   std::atomic<unsigned long long> ctx[8] = {};
+};
+// Allow `kern` maxSmem bytes of dynamic shared memory in the current context; called before every launch
+// that needs more than 48 KB. (Raised before each launch, not once per context, a call costs 0.5 us more:
+// 64^3 FP32, one threshold 28.3 -> 28.8 us.)
+template <typename K>
+void allowSmem(SmemAllowed &done, K kern, size_t maxSmem)
+{
+   const unsigned long long id = contextId();
+   std::atomic<unsigned long long> &slot = done.ctx[id % 8];
+   if (id != 0 && slot.load(std::memory_order_relaxed) == id) { return; }
+   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)maxSmem) == cudaSuccess) {
+      slot.store(id, std::memory_order_relaxed);
+   }
 }
 // Resident CTAs per SM of `kern` for a block size and dynamic shared-memory size (allowSmem beforehand
 // above 48 KB), computed on the first call for a cache slot and kept there (a relaxed atomic: host

@@ -313,7 +313,8 @@ static int launchThermoT(const FusedArgs &a, cudaStream_t s)
 {
    static std::atomic<int> occ[MKF_MAX_THRESH + 1];  // resident CTAs for each K's histogram size
    auto kern = thermoBPFD<T, TY, GE, INNER, CMAX>;
-   allowSmem(kern, thermoDynBytes(MKF_MAX_THRESH));
+   static SmemAllowed allowed;
+   allowSmem(allowed, kern, thermoDynBytes(MKF_MAX_THRESH));
    const int blocksPerSM = cachedOccupancy(occ[a.K], kern, kThWarps * 32, thermoDynBytes(a.K));
    long long grid = (a.nItems + kThWarps - 1) / kThWarps;
    const long long cap = (long long)smCount() * blocksPerSM;
@@ -401,7 +402,8 @@ static int launchThermoBatchV(const BatchArgs &b, int maxK, cudaStream_t s)
    static std::atomic<int> occ[MKF_MAX_THRESH + 1];
    auto kern = thermoBatch<T, TY, V>;
    const size_t smem = thermoDynBytes(maxK);  // every field of the group has at most maxK thresholds
-   allowSmem(kern, thermoDynBytes(MKF_MAX_THRESH));
+   static SmemAllowed allowed;
+   allowSmem(allowed, kern, thermoDynBytes(MKF_MAX_THRESH));
    const int blocksPerSM = cachedOccupancy(occ[maxK], kern, kThWarps * 32, smem);
    long long grid = (long long)smCount() * blocksPerSM;
    if (grid > b.nChunks) { grid = b.nChunks; }

@@ -652,7 +652,8 @@ static int launchTmaN(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
    static std::atomic<int> occ[kTmMaxK + 1];
    auto kern = thermoTmaBPFD<T, GE, CMAX, V, COPY, NS>;
    const size_t smem = tmaDynBytes<T, V>(a.K);
-   allowSmem(kern, tmaDynBytes<T, V>(kTmMaxK));
+   static SmemAllowed allowed;
+   allowSmem(allowed, kern, tmaDynBytes<T, V>(kTmMaxK));
    const int blocksPerSM = cachedOccupancy(occ[a.K], kern, G::WARPS * 32, smem);
    long long grid = (a.nItems + G::WARPS - 1) / G::WARPS;
    const long long cap = (long long)smCount() * blocksPerSM;

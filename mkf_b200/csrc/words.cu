@@ -113,8 +113,9 @@ static void wordGrid(const WordTask &a, int enc, bool mis, int ctas, int &depth,
 template <typename T, bool MOM, int KT, bool MIS>
 static int launchWordsT(WordTask &a, int enc, cudaStream_t s)
 {
+   static SmemAllowed allowed;
    auto kern = wordBPFD<T, MOM, KT, MIS>;
-   allowSmem(kern, kWdDynBytes);
+   allowSmem(allowed, kern, kWdDynBytes);
    int depth, strip;
    wordGrid(a, enc, MIS, smCount(), depth, strip);
    if (!MOM) { depth = tunedDepth(kFamWords, enc, a.K, a.X, a.Y, a.Z, depth); }

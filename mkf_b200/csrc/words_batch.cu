@@ -61,8 +61,9 @@ std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks)
 template <typename T>
 static int launchBatchT(const WordBatchArgs &b, cudaStream_t s)
 {
+   static SmemAllowed allowed;
    auto kern = wordBatch<T>;
-   allowSmem(kern, kWdDynBytes);
+   allowSmem(allowed, kern, kWdDynBytes);
    long long grid = smCount();
    if (grid > b.nChunks) { grid = b.nChunks; }
    if (grid < 1) { grid = 1; }
