@@ -19,6 +19,7 @@
 //   * rows shorter than 32 elements contribute X-1 cells (the original counts 2X-1).
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include "mkf_common.cuh"
 #include "binMapCUDA.h"
 #include "mkfCUDA.h"
@@ -256,46 +257,90 @@ static size_t *gBPFDHost = nullptr;
 
 static size_t *gBPFDStage = nullptr;  // pinned: counts on their way to the caller's array
 
-// Stage timer of the original's interface. The two events belong to the calling thread and device and
-// are kept between calls (creating and destroying them cost 4 us of each call).
+// Pairs of timing events that no call is using. A pair belongs to the context that it was made in (a
+// reset of the device ends that context and its events) and is used in it only. At most kEventPairs are
+// kept, and the clean-up functions give the current context's back.
+struct EventPair
+{
+   unsigned long long ctx;
+   cudaEvent_t e0, e1;
+};
+static constexpr int kEventPairs = 16;
+static std::mutex gEventMu;
+static EventPair gEvents[kEventPairs];
+static int gNumEvents = 0;
+
+static void destroyEvents(const EventPair &p)
+{
+   if (p.e0) { cudaEventDestroy(p.e0); }
+   if (p.e1) { cudaEventDestroy(p.e1); }
+}
+
+static EventPair takeEvents()
+{
+   const unsigned long long ctx = contextId();
+   {
+      std::lock_guard<std::mutex> lk(gEventMu);
+      for (int i = 0; i < gNumEvents && ctx != 0; i++) {
+         if (gEvents[i].ctx == ctx) {
+            const EventPair p = gEvents[i];
+            gEvents[i] = gEvents[--gNumEvents];
+            return p;
+         }
+      }
+   }
+   EventPair p = {ctx, nullptr, nullptr};
+   cudaEventCreate(&p.e0);
+   cudaEventCreate(&p.e1);
+   return p;
+}
+
+static void giveEvents(const EventPair &p)
+{
+   if (p.ctx != 0 && p.e0 && p.e1) {
+      std::lock_guard<std::mutex> lk(gEventMu);
+      if (gNumEvents < kEventPairs) {
+         gEvents[gNumEvents++] = p;
+         return;
+      }
+   }
+   destroyEvents(p);
+}
+
+static void dropEvents()
+{
+   const unsigned long long ctx = contextId();
+   std::lock_guard<std::mutex> lk(gEventMu);
+   int n = 0;
+   for (int i = 0; i < gNumEvents; i++) {
+      if (gEvents[i].ctx == ctx) { destroyEvents(gEvents[i]); }
+      else { gEvents[n++] = gEvents[i]; }
+   }
+   gNumEvents = n;
+}
+
+// Stage timer of the original's interface (events made and destroyed by each call instead of kept:
+// 68.0 -> 69.5 us for the pair of calls on a 256^3 map).
 class EventTimer
 {
  public:
-   EventTimer() { cudaEventRecord(ev().e0, 0); }
-   void mark() { cudaEventRecord(ev().e1, 0); }
+   EventTimer() : ev_(takeEvents()) { cudaEventRecord(ev_.e0, 0); }
+   ~EventTimer() { giveEvents(ev_); }
+   EventTimer(const EventTimer &) = delete;
+   EventTimer &operator=(const EventTimer &) = delete;
+   void mark() { cudaEventRecord(ev_.e1, 0); }
    // wait for the mark (or for work issued after it on the stream: one wait for both) and read the time
-   float stop(bool stream = false) {
+   float stop(bool stream = false)
+   {
       float ms = 0;
       if (stream) { cudaStreamSynchronize(0); }
-      else { cudaEventSynchronize(ev().e1); }
-      cudaEventElapsedTime(&ms, ev().e0, ev().e1);
+      else { cudaEventSynchronize(ev_.e1); }
+      cudaEventElapsedTime(&ms, ev_.e0, ev_.e1);
       return ms;
    }
 
  private:
-   struct Events
-   {
-      int dev = -1;
-      cudaEvent_t e0 = nullptr, e1 = nullptr;
-      void drop() {
-         if (e0) { cudaEventDestroy(e0); }
-         if (e1) { cudaEventDestroy(e1); }
-         e0 = e1 = nullptr;
-      }
-      ~Events() { drop(); }
-   };
-   static Events &ev() {
-      static thread_local Events e;
-      int dev = 0;
-      cudaGetDevice(&dev);
-      if (e.dev != dev || !e.e0 || !e.e1) {
-         e.drop();
-         cudaEventCreate(&e.e0);
-         cudaEventCreate(&e.e1);
-         e.dev = dev;
-      }
-      return e;
-   }
+   EventPair ev_;
 };
 
 }  // namespace mkf
@@ -384,6 +429,7 @@ MKF_API BMPackWord *binMapCUDA(KernInfo *pK, BMPackWord *pW, BMOrg *pO, const BM
 MKF_API void binMapCUDACleanup(void)
 {
    if (gMap) { cudaFree(gMap); gMap = nullptr; gMapWords = 0; }
+   dropEvents();
 }
 
 MKF_API size_t *mkfCUDAGetBPFD(KernInfo *pK, size_t *pBPFD, const BMOrg *pO, const BMPackWord *pW, const int profile)
@@ -433,6 +479,7 @@ MKF_API void mkfCUDACleanup(int lvl)
    if (gBPFDHost) { cudaFreeHost(gBPFDHost); gBPFDHost = nullptr; }
    if (gBPFDDev) { cudaFree(gBPFDDev); gBPFDDev = nullptr; }
    if (gBPFDStage) { cudaFreeHost(gBPFDStage); gBPFDStage = nullptr; }
+   dropEvents();
 }
 
 MKF_API int mkfCUDAGetBPFDautoCtx(Context *pC, const FieldDef def[3], const BinMapF64 *pM, const int profile)

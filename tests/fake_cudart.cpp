@@ -37,7 +37,7 @@ static void count(const char *what) { std::lock_guard<std::mutex> lk(mu); calls[
 // ---- for the tests
 int fake_calls(const char *what) { std::lock_guard<std::mutex> lk(mu); return calls[what]; }
 int fake_events_alive() { std::lock_guard<std::mutex> lk(mu); return (int)events.size(); }
-// The launched kernels since the last call, one per line: device, name, dynamic shared memory.
+// The launched kernels since the last call, one per line: device, name, dynamic shared memory, blocks, threads.
 const char *fake_launches()
 {
    static std::string s;
@@ -73,7 +73,8 @@ Err cudaLaunchKernel(const void *f, Dim3 g, Dim3 b, void **, size_t smem, void *
 {
    std::lock_guard<std::mutex> lk(mu);
    if (smem > limitOf(f) || g.x == 0 || b.x == 0 || b.x > 1024) { return fail(BAD_VALUE); }
-   launches.push_back(std::to_string(curDev) + " " + kernelName[f] + " " + std::to_string(smem));
+   launches.push_back(std::to_string(curDev) + " " + kernelName[f] + " " + std::to_string(smem) + " " +
+                      std::to_string(g.x) + " " + std::to_string(b.x));
    return OK;
 }
 Err cudaFuncSetAttribute(const void *f, int attr, int v)

@@ -95,3 +95,69 @@ calls("before")
 assert fake.cudaDeviceReset() == 0
 calls("after")
 """)
+
+
+def test_map_and_count_after_clean_up_and_reset(fake):
+    """The original's pair: its callers clean up (the original resets the device there) and count on."""
+    fake(r"""
+import threading
+m = _lib.BinMapF64()
+lib.setBinMapF64(C.byref(m), b">", 0.0)
+table = (_lib.ConstFieldPtr * 4)()
+table[0].p = data.ctypes.data
+fi = _lib.BMFieldInfo()
+fi.fieldTableMask, fi.elemID, fi.profID = 1, M.ENC_F32, 0
+defs = (C.c_int * 3)(64, 40, 40)
+fi.pD = defs
+fi.pFieldDevPtrTable = table
+
+def pair(where, own=None):
+    org, ki, host = _lib.BMOrg(), _lib.KernInfo(), np.zeros(256, np.uint64)
+    p = lib.binMapCUDA(C.byref(ki), own, C.byref(org), C.byref(fi), C.byref(m))
+    assert p, (where, "map")
+    assert ki.dtms[0] == 0.25, (where, ki.dtms[0])
+    assert lib.mkfCUDAGetBPFD(C.byref(ki), data.ctypes.data, C.byref(org), p, 0), (where, "count")
+    assert lib.mkfCUDAGetBPFDH(C.byref(ki), host.ctypes.data, C.byref(org), p, 0), (where, "count to host")
+    assert ki.dtms[1] == 0.25, (where, ki.dtms[1])
+    names = [l[1] for l in launches()]
+    assert sum("countMap" in n for n in names) == 2, (where, names)
+
+def clean():
+    lib.mkfCUDACleanup(1)
+    lib.binMapCUDACleanup()
+
+pair("first")
+pair("second")
+clean()
+pair("after clean-up")
+clean()
+assert fake.cudaDeviceReset() == 0
+pair("after clean-up and reset")
+assert fake.cudaSetDevice(1) == 0
+clean()
+pair("second device")
+clean()
+assert fake.cudaSetDevice(0) == 0
+clean()
+assert fake.cudaDeviceReset() == 0
+t = threading.Thread(target=lambda: pair("thread"))
+t.start()
+t.join()
+assert fake.fake_calls(b"dead event") == 0
+# a caller's own buffers and no clean-up: the count needs nothing that a reset takes
+org, ki = _lib.BMOrg(), _lib.KernInfo()
+own = np.zeros(1 << 16, np.uint32)
+assert lib.binMapCUDA(C.byref(ki), own.ctypes.data, C.byref(org), C.byref(fi), C.byref(m))
+assert fake.cudaDeviceReset() == 0
+assert lib.binMapCUDA(C.byref(ki), own.ctypes.data, C.byref(org), C.byref(fi), C.byref(m))
+assert lib.mkfCUDAGetBPFD(C.byref(ki), data.ctypes.data, C.byref(org), own.ctypes.data, 0)
+for i in range(40):
+    assert lib.mkfCUDAGetBPFD(C.byref(ki), data.ctypes.data, C.byref(org), own.ctypes.data, 0)
+    assert fake.cudaDeviceReset() == 0
+for i in range(10):
+    assert lib.mkfCUDAGetBPFD(C.byref(ki), data.ctypes.data, C.byref(org), own.ctypes.data, 0)
+assert fake.fake_events_alive() <= 2
+assert fake.fake_calls(b"dead event") == 0
+clean()
+assert fake.fake_events_alive() == 0, fake.fake_events_alive()
+""")
