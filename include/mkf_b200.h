@@ -188,8 +188,9 @@ int mkfServerDestroy(MKFServer *server);
  * item: halo re-reads against work items per SM) and, for the TMA-staged rank-table kernel, a
  * variant of CTA shape and histogram privatisation (0: 20 warps per CTA, two-stage FP64 tile rings,
  * two histogram copies; 1: 16 warps, three stages, two copies; 2: 20 warps, two stages, one copy).
- * A kind of field is the kernel, the element type, the threshold count and the power-of-two size
- * class of each extent (so the row width class too).
+ * A kind of field is the kernel and its way of reading the field (rows on 16-byte boundaries, other
+ * rows, strided x), the element type, the threshold count and the power-of-two size class of each
+ * extent (so the row width class too).
  * mkfTune times the candidate depths (and variants) on this field with these thresholds (the
  * counting runs several times; synchronous) and keeps the fastest for fields of the same kind;
  * later mkfFieldBPFD calls on such fields use it; without tuning each kernel uses its default.

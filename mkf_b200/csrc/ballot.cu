@@ -287,7 +287,7 @@ int launchBallots(WordTask &a, int enc, cudaStream_t s)
 {
    a.nStripX = (a.X - 1 + 30) / 31;
    a.nTileY = (a.Y - 1 + 30) / 31;
-   a.D = tunedDepth(kFamWords, enc, a.K, a.X, a.Y, a.Z,
+   a.D = tunedDepth(kFamBallot, enc, a.K, a.X, a.Y, a.Z,
                     sizeDepth(kBlD, (long long)a.nStripX * a.nTileY, a.Z, (long long)smCount() * kBlItemsPerSM));
    a.nSlabZ = (a.Z - 1 + a.D - 1) / a.D;
    a.nItems = (long long)a.nStripX * a.nTileY * a.nSlabZ;

@@ -145,8 +145,12 @@ int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, Fie
                    std::vector<ConstEntry> &consts, bool &anyVarying, int depth = 0);
 
 // Slab depth (planes of cells per work item) of a single-field launch of kernel family `family`
-// (tune.cu): the depth mkfTune measured best for this kind of field, else `def`.
-enum { kFamWords = 0, kFamThermo = 1, kFamThermoTma = 2 };
+// (tune.cu): the depth mkfTune measured best for this kind of field, else `def`. A family is one kernel
+// with one way of reading the field, so that what was measured on it is used by it only: the word kernel
+// on aligned rows, on others and with strided x; the vote kernel; the rank table read from global memory;
+// the staged rank table filled by TMA (also with thresholds sharing buckets), by blocks and by elements.
+enum { kFamWords, kFamWordsBlocks, kFamWordsElems, kFamBallot, kFamThermo, kFamThermoTma, kFamThermoTmaShared,
+       kFamThermoBlocks, kFamThermoElems, kNumFamilies };
 static constexpr int kTmNumVariants = 4;  // variants of the TMA rank-table kernel (thermo_tma.cu)
 int tunedDepth(int family, int enc, int K, int X, int Y, int Z, int def);
 // Kernel variant (CTA shape, histogram copies) of such a launch: the one mkfTune measured best for

@@ -487,8 +487,9 @@ int launchThermo(FusedArgs &a, int enc, cudaStream_t s)
    const long long perPlane = (long long)((a.X - 1 + 30) / 31) * ((a.Y - 1 + THERMO_TY - 1) / THERMO_TY);
    // up to 16 thresholds on fields of at least one tile: tiles staged in shared memory
    if (thermoRingEligible(a)) {
-      itemGrid(a, tunedDepth(kFamThermoTma, enc, a.K, a.X, a.Y, a.Z, ringDepth(perPlane, a.Z - 1, (long long)smCount() * kTmWarpsPerSM)));
-      const int rc = launchThermoRing(a, enc, tunedVariant(kFamThermoTma, enc, a.K, a.X, a.Y, a.Z, 0), s);
+      const int family = thermoRingFamily(a, enc);
+      itemGrid(a, tunedDepth(family, enc, a.K, a.X, a.Y, a.Z, ringDepth(perPlane, a.Z - 1, (long long)smCount() * kTmWarpsPerSM)));
+      const int rc = launchThermoRing(a, enc, tunedVariant(family, enc, a.K, a.X, a.Y, a.Z, 0), s);
       if (rc != MKF_ERR_UNSUPPORTED) { return rc; }
    }
    itemGrid(a, tunedDepth(kFamThermo, enc, a.K, a.X, a.Y, a.Z,

@@ -329,6 +329,7 @@ __device__ __forceinline__ uint32_t cellCode(uint32_t R0, uint32_t R1, uint32_t 
 // pass (after prepareKeys), and its launch (after itemGrid; MKF_ERR_UNSUPPORTED when it does not).
 static constexpr int kTmWarpsPerSM = 20;  // resident warps of the default variant
 bool thermoRingEligible(const FusedArgs &a);
+int thermoRingFamily(const FusedArgs &a, int enc);  // the tuning family of its launch
 // variant: CTA shape, histogram privatisation and queue kind (kTmVariants in thermo_tma.cu,
 // kTmNumVariants of them), 0 = default; fields off 16-byte boundaries have the default only.
 int launchThermoRing(const FusedArgs &a, int enc, int variant, cudaStream_t s);

@@ -711,6 +711,12 @@ bool thermoRingEligible(const FusedArgs &a)
    return a.K > 2 && a.K <= kTmMaxK && a.X >= 32 && a.Y >= 9 && a.Z >= 2 && a.lutC >= 1;
 }
 
+int thermoRingFamily(const FusedArgs &a, int enc)
+{
+   if (tmaRowsAligned(a, enc)) { return a.lutC > 1 ? kFamThermoTmaShared : kFamThermoTma; }
+   return a.sx == 1 ? kFamThermoBlocks : kFamThermoElems;
+}
+
 // a.tkey / a.lutC filled (prepareKeys) and the item grid set for 8-row items (itemGrid).
 int launchThermoRing(const FusedArgs &a, int enc, int variant, cudaStream_t s)
 {

@@ -5,8 +5,9 @@
 // ones give small fields enough work items to fill 148 SMs. The TMA-staged rank-table kernel also
 // comes in variants of CTA shape (warps per CTA with the depth of their tile rings) and histogram
 // privatisation (one or two copies). mkfTune times the candidates on a caller's field and
-// remembers the fastest for fields of the same kind (kernel family, element type, threshold count,
-// and the power-of-two size class of each extent, which includes the row width); later
+// remembers the fastest for fields of the same kind (kernel family, which includes the way rows are
+// read, element type, threshold count, and the power-of-two size class of each extent, which includes
+// the row width); later
 // single-field calls on such fields use it. Batch plans time whole candidate plans when they are
 // created (mkfSetTuning switches that off).
 #include <algorithm>
@@ -39,7 +40,8 @@ static int log2Class(int n)
    return b;
 }
 
-static constexpr int kVariantsOf[3] = {1, 1, kTmNumVariants};  // variants per family (words, rank table, TMA rank table)
+// Variants of a kernel family.
+static constexpr int variantsOf(int family) { return family == kFamThermoTma ? kTmNumVariants : 1; }
 
 static std::mutex gTuneMu;
 static std::map<TuneKey, TuneVal> gTuned;
@@ -66,7 +68,7 @@ int tunedDepth(int family, int enc, int K, int X, int Y, int Z, int def)
 
 int tunedVariant(int family, int enc, int K, int X, int Y, int Z, int def)
 {
-   const int nv = (family >= 0 && family < 3) ? kVariantsOf[family] : 1;
+   const int nv = variantsOf(family);
    if (tForceVariant >= 0) { return tForceVariant < nv ? tForceVariant : 0; }
    std::lock_guard<std::mutex> lk(gTuneMu);
    auto it = gTuned.find(keyOf(family, enc, K, X, Y, Z));
@@ -141,7 +143,7 @@ MKF_API int mkfTune(const MKFFieldDesc *pF, const MKFThreshSet *pT, void *stream
    float ms = 0.0f;
    if (rc == MKF_OK) { rc = runOnce(pF, pT, tmp, s, kCand[0], 0, &seen, 0, e0, e1, &ms); }
    int nVar = 1;
-   for (const TuneKey &k : seen) { nVar = std::max(nVar, (k.family >= 0 && k.family < 3) ? kVariantsOf[k.family] : 1); }
+   for (const TuneKey &k : seen) { nVar = std::max(nVar, variantsOf(k.family)); }
    float best = 0.0f;
    int bestD = 0, bestV = 0;
    for (int v = 0; v < nVar && rc == MKF_OK; v++) {
@@ -156,7 +158,7 @@ MKF_API int mkfTune(const MKFFieldDesc *pF, const MKFThreshSet *pT, void *stream
    }
    if (rc == MKF_OK && bestD > 0) {
       std::lock_guard<std::mutex> lk(gTuneMu);
-      for (const TuneKey &k : seen) { gTuned[k] = TuneVal{bestD, k.family < 3 && bestV < kVariantsOf[k.family] ? bestV : 0}; }
+      for (const TuneKey &k : seen) { gTuned[k] = TuneVal{bestD, bestV < variantsOf(k.family) ? bestV : 0}; }
    }
    if (tmp) { cudaFree(tmp); }
    if (e0) { cudaEventDestroy(e0); }
@@ -181,7 +183,7 @@ MKF_API int mkfTuneSet(const MKFFieldDesc *pF, const MKFThreshSet *pT, int depth
       std::lock_guard<std::mutex> lk(gTuneMu);
       for (const TuneKey &k : seen) {
          if (depth > 0) {
-            gTuned[k] = TuneVal{depth, k.family < 3 && variant < kVariantsOf[k.family] ? variant : 0};
+            gTuned[k] = TuneVal{depth, variant < variantsOf(k.family) ? variant : 0};
          } else {
             gTuned.erase(k);
          }

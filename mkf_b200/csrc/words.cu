@@ -71,7 +71,8 @@ static int wordWarps(int enc, int K, int W, bool mis)
    return std::min(kWdWarps, kWdDynBytes / wordWarpBytes(enc == ENC_F32 ? 4 : 2, K, W, mis));
 }
 
-static void wordGrid(const WordTask &a, int enc, bool mis, int ctas, int &depth, int &strip)
+// Planes per work item and tiles per strip; tuned: the planes are given (0: chosen too).
+static void wordGrid(const WordTask &a, int enc, bool mis, int ctas, int tuned, int &depth, int &strip)
 {
    // Cost of a grid, fitted to sweeps of depth and strip over 256^3 to 128 x 2048^2 fields with one
    // and three thresholds (the choice is within 5 % of the best swept). The busiest warp's tiles:
@@ -90,17 +91,23 @@ static void wordGrid(const WordTask &a, int enc, bool mis, int ctas, int &depth,
       const int strips = (chunks + w - 1) / w, W = (chunks + strips - 1) / strips;
       const int perCta = wordWarps(enc, a.K, W, mis);
       const long long warps = (long long)ctas * perCta;
-      for (int r = 1; r <= 16; r++) {
-         // the shallowest slabs that r rounds take
-         const long long slabs = std::min<long long>(cellsZ, r * warps / (strips * tiles));
-         if (slabs < 1) { continue; }
-         const int d = (int)((cellsZ + slabs - 1) / slabs);
+      auto consider = [&](long long r, int d) {
          const double cost = (double)r * ((d + 1) * W + 1) * (1.0 + burst / W) * std::sqrt((double)perCta / kWdWarps);
-         if (d <= kWordMaxDepth && (best == 0.0 || cost < best)) {
+         if (best == 0.0 || cost < best) {
             best = cost;
             depth = d;
             strip = W;
          }
+      };
+      if (tuned > 0) {
+         consider((strips * tiles * ((cellsZ + tuned - 1) / tuned) + warps - 1) / warps, tuned);
+      }
+      for (int r = 1; r <= 16 && tuned == 0; r++) {
+         // the shallowest slabs that r rounds take
+         const long long slabs = std::min<long long>(cellsZ, r * warps / (strips * tiles));
+         if (slabs < 1) { continue; }
+         const int d = (int)((cellsZ + slabs - 1) / slabs);
+         if (d <= kWordMaxDepth) { consider(r, d); }
       }
       if (w == 1) { break; }
    }
@@ -117,8 +124,8 @@ static int launchWordsT(WordTask &a, int enc, cudaStream_t s)
    auto kern = wordBPFD<T, MOM, KT, MIS>;
    allowSmem(allowed, kern, kWdDynBytes);
    int depth, strip;
-   wordGrid(a, enc, MIS, smCount(), depth, strip);
-   if (!MOM) { depth = tunedDepth(kFamWords, enc, a.K, a.X, a.Y, a.Z, depth); }
+   const int family = MIS ? kFamWordsBlocks : a.vec ? kFamWords : kFamWordsElems;
+   wordGrid(a, enc, MIS, smCount(), MOM ? 0 : tunedDepth(family, enc, a.K, a.X, a.Y, a.Z, 0), depth, strip);
    fillWordGrid(a, enc, depth, strip);
    const int warps = wordWarps(enc, a.K, a.W, MIS);
    const long long grid = std::min<long long>((a.nItems + warps - 1) / warps, smCount());

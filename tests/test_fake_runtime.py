@@ -161,3 +161,86 @@ assert fake.fake_calls(b"dead event") == 0
 clean()
 assert fake.fake_events_alive() == 0, fake.fake_events_alive()
 """)
+
+
+def test_a_tuned_depth_belongs_to_one_kernel(fake):
+    """Fields of one size class that different kernels or ways of copying count: a depth and variant
+    recorded for one leaves the others alone."""
+    fake(r"""
+def desc(dt, shape, kind):
+    Z, Y, X = shape
+    if kind == "aligned":
+        return field(shape, dt)
+    if kind == "odd":
+        return field(shape, dt, 1, (Y * (X + 1), X + 1, 1))
+    return field(shape, dt, 0, (2 * Y * X, 2 * X, 2))
+
+def query(d, th):
+    dep, var = C.c_int(-1), C.c_int(-1)
+    assert lib.mkfTuneQuery(C.byref(d), C.byref(th.ts), C.byref(dep), C.byref(var), None) == 0
+    return dep.value, var.value
+
+for dt in (np.float32, np.float64):
+    # (nothing reads the fields here, so they may be larger than the memory behind them)
+    for shape, ks in (((40, 40, 64), (1, 2, 3, 6, 12, 16)), ((260, 260, 272), (2, 3, 4, 5, 8)), ((520, 520, 544), (1, 2, 5))):
+        for k in ks:
+            sets = {"spread": M._Thresholds(list(np.linspace(-1.0, 1.0, k)), 4)}
+            if 2 < k <= 4 or 4 < k <= 16:
+                sets["shared"] = M._Thresholds([100.0 + 1e-3 * i if i < 3 else 200.0 * i for i in range(k)], 4)
+            kinds = {}  # what launches -> the descriptions that launch it
+            for kind in ("aligned", "odd", "strided"):
+                for tn, th in sets.items():
+                    d = desc(dt, shape, kind)
+                    out = np.zeros((k, 256), np.uint64)
+                    launches()
+                    assert lib.mkfFieldBPFD(out.ctypes.data, C.byref(d), C.byref(th.ts), 0, None) == 0
+                    name = launches()[-1][1]
+                    name = name.split("BPFD")[0]
+                    if "ballot" in name or name.endswith("thermo"):  # read any field alike
+                        kinds.setdefault((name, "", ""), []).append((d, th))
+                    else:  # (a threshold set sharing buckets has no variants to choose from)
+                        kinds.setdefault((name, kind, tn if "thermoTma" in name and kind == "aligned" else ""), []).append((d, th))
+            for me, mine in kinds.items():
+                d, th = mine[0]
+                variant = 3 if "thermoTma" in me[0] and me[1] == "aligned" and me[2] == "spread" else 0
+                assert lib.mkfTuneSet(C.byref(d), C.byref(th.ts), 24, 3, None) == 0
+                assert query(d, th) == (24, variant), (me, query(d, th))
+                for other, theirs in kinds.items():
+                    if other != me:
+                        for d2, th2 in theirs:
+                            assert query(d2, th2) == (0, 0), (shape, k, me, other)
+                assert lib.mkfTuneSet(C.byref(d), C.byref(th.ts), 0, 0, None) == 0
+                assert query(d, th) == (0, 0)
+""")
+
+
+def test_a_tuned_depth_gets_its_own_strips(fake):
+    """The word kernel's strips for a recorded depth are those that suit it: by the cost that words.cu
+    chooses strips by, none is worse than strips of one tile."""
+    fake(r"""
+def grid(d, th):
+    out = np.zeros((th.n, 256), np.uint64)
+    assert lib.mkfFieldBPFD(out.ctypes.data, C.byref(d), C.byref(th.ts), 0, None) == 0
+    name, smem, blocks, threads = launches()[-1][1:5]
+    assert "wordBPFD" in name
+    return int(smem), int(blocks), int(threads) // 32
+
+th = M._Thresholds([-0.5, 0.0, 0.5], [4, 1, 2])
+for shape in ((64, 512, 1024), (128, 256, 512), (33, 700, 2048)):
+    d = field(shape, np.float32)
+    for depth in (4, 16, 64, 128):
+        assert lib.mkfTuneSet(C.byref(d), C.byref(th.ts), depth, 0, None) == 0
+        smem, blocks, warps = grid(d, th)
+        W = (smem // warps - 2 * 32 * 144 - 9 * 288) // 128  # state words: 3 (2 W + 3)
+        W = (W // 3 - 3) // 2
+        tiles, rows, slabs = -(-(shape[2] - 1) // 32), -(-(shape[1] - 1) // 31), -(-(shape[0] - 1) // depth)
+
+        burst = 0.7 / 3 if 128 * tiles * shape[1] * shape[0] > 32e6 else 0.0
+
+        def cost(W, warps):
+            rounds = -(-(-(-tiles // W) * rows * slabs) // (148 * warps))
+            return rounds * ((depth + 1) * W + 1) * (1 + burst / W) * (warps / 16) ** 0.5
+
+        assert cost(W, warps) <= 1.0001 * cost(1, 16), (shape, depth, W)
+        assert lib.mkfTuneSet(C.byref(d), C.byref(th.ts), 0, 0, None) == 0
+""")
