@@ -37,6 +37,7 @@
 #include <cstring>
 #include <mutex>
 #include "thermo.cuh"
+#include "blocks.cuh"
 #include "tma.cuh"
 
 namespace mkf {
@@ -55,7 +56,6 @@ struct TmaVariant
 };
 static constexpr TmaVariant kTmVariants[kTmNumVariants] = {{20, 2, 3, 2, 1}, {16, 3, 4, 2, 0}, {20, 2, 3, 1, 1},
                                                            {20, 2, 3, 2, 0}};
-static constexpr int kTmRows = 9;           // rows of a plane tile: 8 row pairs
 // wide-cell queue entries per warp: a plane adds at most 8 x 31, drained once 32 are waiting (plus
 // one discard entry)
 static constexpr int kTmQueue = 32 + 8 * 31;  // drained after a plane once 32 are waiting
@@ -218,39 +218,8 @@ __device__ __forceinline__ void drainLanes(const uint2 *qw, int n, uint32_t hist
    __syncwarp();
 }
 
-// Geometry of one work item: 31 x positions of cells, 8 row pairs, up to D planes of cells.
-struct TmItem
-{
-   int xa, xoff;     // tile x (a multiple of ALIGN) and this item's first lane column in it
-   int y0, z0, nPln; // tile rows y0 .. y0 + 8, planes z0 .. z0 + nPln
-   uint32_t rowsOK;  // bit j: this lane counts row pair j
-   unsigned cells;   // cells the item counts (warp total)
-};
-
-template <int ALIGN>
-__device__ __forceinline__ TmItem itemOf(const FusedArgs &a, long long it, int lane)
-{
-   TmItem m;
-   const int ix = (int)(it % a.nSegX);
-   const long long rest = it / a.nSegX;
-   const int iy = (int)(rest % a.nTileY);
-   const int iz = (int)(rest / a.nTileY);
-   const int xs = 31 * ix, ys = 8 * iy;
-   const int xe = min(xs + 31, a.X - 1), ye = min(ys + 8, a.Y - 1);
-   const int x0 = min(xs, a.X - 32);  // lanes at x0 + lane, all inside the field
-   m.xa = x0 & ~(ALIGN - 1);
-   m.xoff = x0 - m.xa;
-   m.y0 = min(ys, a.Y - 9);
-   m.z0 = a.D * iz;
-   m.nPln = min(a.D, a.Z - 1 - m.z0);
-   const int jlo = ys - m.y0, jhi = ye - m.y0;
-   const bool laneIn = x0 + lane >= xs && x0 + lane < xe;
-   m.rowsOK = laneIn ? (((1u << jhi) - 1u) & ~((1u << jlo) - 1u)) : 0u;
-   m.cells = (unsigned)(xe - xs) * (unsigned)(jhi - jlo) * (unsigned)m.nPln;
-   return m;
-}
-
-// COPY: how the ring is filled. Fields that a tensor map cannot take use cp.async: with strided x every
+// COPY: how the ring is filled. Fields that a tensor map cannot take use cp.async: with strided x, or rows or
+// planes that lie backwards or less than a block apart, every
 // lane copies its own column of the tile, one element per row, and waits for its own copies only; where
 // only the alignment of the rows is off, the warp copies the 16-byte blocks that the rows touch, and a
 // row is read from where it starts in its first block. The rest is the same. Against thermo.cu, which took these fields
@@ -265,9 +234,7 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    using G = TmaGeom<T, V>;
    constexpr bool TMA = COPY == kCopyTma;
    constexpr int B = (int)sizeof(T), ROWB = G::BX * B;  // bytes of an element, of a tile row
-   constexpr int NB = 2 * B;                            // blocks of a row of 32 elements
-   constexpr int NR = 32 / NB;                          // rows per copy of blocks
-   static_assert(ROWB == 16 * (NB + 1) && 8 % NR == 0 && NB + kTmRows <= 32, "rows of NB + 1 blocks");
+   static_assert(ROWB == RingBlocks<T>::ROWB, "rows of whole blocks");
    constexpr int kTmWarps = G::WARPS, kHistCopies = G::COPIES;
    constexpr int W = sizeof(T) / 4;   // 32-bit words per element; the ranked word is the last
    constexpr int S = G::STAGES;
@@ -310,9 +277,9 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
    // producer cursor (every lane tracks it; lane 0 issues): item, plane, tile coordinates
    long long pIt = first;
    int pP = 0, pX = 0, pY = 0, pZ = 0, pN = -1;
-   // (elements) this lane's element of the tile's first row; (blocks) this lane's block of its row among
-   // the first NR, plus the row's offset in a block
-   const char *pCol = nullptr;
+   const char *pCol = nullptr;  // (elements) this lane's element of the tile's first row
+   RingBlocks<T> blocks;
+   bool tail = false;  // (blocks) the last plane of the field's last item is still to be copied
    auto begin = [&]() {
       if (pIt < a.nItems) {
          const TmItem m = itemOf<G::ALIGN>(a, pIt, lane);
@@ -321,8 +288,12 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
             pCol = (const char *)a.f + ((int64_t)(m.xa + m.xoff + lane) * a.sx + (int64_t)m.y0 * a.sy + (int64_t)m.z0 * a.sz) * (int64_t)B;
          }
          if (COPY == kCopyBlocks) {
-            pCol = (const char *)a.f + ((int64_t)(m.xa + m.xoff) + (int64_t)(m.y0 + lane / NB) * a.sy + (int64_t)m.z0 * a.sz) * (int64_t)B +
-                   16 * (lane % NB);
+            blocks.begin(a, m, lane);
+            // (no item of this warp comes after it: the last two items are another warp's each)
+            if (RingBlocks<T>::atLast(a, m)) {
+               tail = true;
+               --pN;
+            }
          }
       }
    };
@@ -343,22 +314,7 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
             }
             pCol += a.sz * (int64_t)B;
          } else {
-            // NB blocks of NR rows at a time; then the ninth row's and, by the next nine lanes, each row's
-            // last block, which it touches only where it does not start on a boundary. Every block copied
-            // holds a byte of the field, so it lies in the field's allocation.
-            const uint32_t tile = ringW + st * G::PITCH, dst = tile + (uint32_t)((lane / NB) * ROWB + (lane % NB) * 16);
-            const char *q = pCol;
-#pragma unroll
-            for (int k = 0; k < 8 / NR; ++k) {
-               asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(k * NR * ROWB)), "l"((uintptr_t)q & ~(uintptr_t)15) : "memory");
-               q += a.sy * (int64_t)(NR * B);
-            }
-            const int row = lane < NB ? 8 : lane - NB, blk = lane < NB ? lane : NB;
-            q = pCol + a.sy * (int64_t)((row - lane / NB) * B) + 16 * (blk - lane % NB);
-            if (lane < NB || (lane < NB + kTmRows && ((uintptr_t)q & 15) != 0)) {
-               asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tile + (uint32_t)(row * ROWB + blk * 16)), "l"((uintptr_t)q & ~(uintptr_t)15) : "memory");
-            }
-            pCol += a.sz * (int64_t)B;
+            blocks.copy(a, ringW + st * G::PITCH, lane);
          }
          ++gp;
          if (++pP > pN) {
@@ -366,6 +322,10 @@ __global__ void __launch_bounds__(kTmVariants[V].warps * 32, 1)
             pP = 0;
             begin();
          }
+      } else if (COPY == kCopyBlocks && tail) {
+         blocks.copyLast(a, ringW + (gp % S) * G::PITCH, lane);
+         ++gp;
+         tail = false;
       }
       if (!TMA) { asm volatile("cp.async.commit_group;" ::: "memory"); }
    };
@@ -688,7 +648,7 @@ static int launchTmaT(const FusedArgs &a, const CUtensorMap &tm, cudaStream_t s)
 template <typename T, bool GE>
 static int launchTmaG(const FusedArgs &a, const CUtensorMap &tm, bool tma, int variant, cudaStream_t s)
 {
-   if (!tma && a.sx == 1) { return a.lutC > 1 ? launchTmaT<T, GE, 4, 0, kCopyBlocks>(a, tm, s) : launchTmaT<T, GE, 1, 0, kCopyBlocks>(a, tm, s); }
+   if (!tma && blockRows(a, (int)sizeof(T))) { return a.lutC > 1 ? launchTmaT<T, GE, 4, 0, kCopyBlocks>(a, tm, s) : launchTmaT<T, GE, 1, 0, kCopyBlocks>(a, tm, s); }
    if (!tma) { return a.lutC > 1 ? launchTmaT<T, GE, 4, 0, kCopyElems>(a, tm, s) : launchTmaT<T, GE, 1, 0, kCopyElems>(a, tm, s); }
    if (a.lutC > 1) { return launchTmaT<T, GE, 4, 0, kCopyTma>(a, tm, s); }
    switch (variant) {
@@ -714,7 +674,7 @@ bool thermoRingEligible(const FusedArgs &a)
 int thermoRingFamily(const FusedArgs &a, int enc)
 {
    if (tmaRowsAligned(a, enc)) { return a.lutC > 1 ? kFamThermoTmaShared : kFamThermoTma; }
-   return a.sx == 1 ? kFamThermoBlocks : kFamThermoElems;
+   return blockRows(a, enc == ENC_F32 ? 4 : 8) ? kFamThermoBlocks : kFamThermoElems;
 }
 
 // a.tkey / a.lutC filled (prepareKeys) and the item grid set for 8-row items (itemGrid).

@@ -31,7 +31,7 @@
 // relations (before: a binary search per element and a loop per map bit) 656 -> 120; moments of
 // 400^3 FP64, 2 thresholds 747 -> 154.
 #pragma once
-#include "fused.cuh"
+#include "blocks.cuh"
 
 namespace mkf {
 
@@ -147,13 +147,6 @@ __device__ inline void rowFlush(const WordTask &a, RowShared &S)
    }
 }
 
-template <int BYTES>
-__device__ __forceinline__ void cpAsync(uint32_t dst, const void *src, int n)
-{
-   if (BYTES == 16) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory"); }
-   else if (BYTES == 8) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory"); }
-   else { asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory"); }
-}
 __device__ __forceinline__ void cpCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cpWait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -174,7 +167,7 @@ struct RowItem
 };
 
 template <int EL>
-__device__ __forceinline__ RowItem rowItemOf(const WordTask &a, long long it)
+__host__ __device__ __forceinline__ RowItem rowItemOf(const WordTask &a, long long it)
 {
    RowItem m;
    int ix, iy, iz;
@@ -202,7 +195,7 @@ __device__ __forceinline__ RowItem rowItemOf(const WordTask &a, long long it)
 // Copies an item's tiles one after another into the warp's ring: 32 rows of EL elements, with the
 // last tile of a strip also the element after each row; rows past the field's last repeat it, elements
 // past the row end are zero.
-template <typename T, bool MIS>
+template <typename T, bool MIS, typename CP = AsyncCopy>
 struct RowCopier
 {
    using G = RowGeom<T, MIS>;
@@ -218,7 +211,7 @@ struct RowCopier
    int nT, tiles, planes; // tiles of a plane; left in the plane, planes left
    bool vec, wide;        // wide: all 32 rows inside, byte offsets below 2^32
 
-   __device__ __forceinline__ void begin(const WordTask &a, const RowItem &m, int lane)
+   __host__ __device__ __forceinline__ void begin(const WordTask &a, const RowItem &m, int lane)
    {
       vec = MIS || a.vec;
       sy = a.sy * B;
@@ -245,21 +238,21 @@ struct RowCopier
          if (nEnd == 0) { step0 = (int64_t)col * a.sx * B; }
       }
    }
-   __device__ __forceinline__ bool left() const { return planes > 0; }
+   __host__ __device__ __forceinline__ bool left() const { return planes > 0; }
    // The 16-byte block of a row whose first byte would be at q (off bytes from the tile's first
-   // element), cut at the row end. A block that holds a byte of the field lies in its allocation.
-   __device__ __forceinline__ void block(uint32_t d, const char *q, int off, bool end)
+   // element), cut at the row end.
+   __host__ __device__ __forceinline__ void block(uint32_t d, const char *q, int off, bool end)
    {
       const uint32_t sh = (uint32_t)(uintptr_t)q & 15u;
       q -= sh;
       if (end) {
          const int n = max(0, min(16, nx * B - off + (int)sh));
-         cpAsync<16>(d, n > 0 ? q : q - off, n);
+         CP::template copy<16>(d, n > 0 ? q : q - off, n);
       } else {
-         cpAsync<16>(d, q, 16);
+         CP::template copy<16>(d, q, 16);
       }
    }
-   __device__ __forceinline__ void copy(uint32_t dst, int lane)
+   __host__ __device__ __forceinline__ void copy(uint32_t dst, int lane)
    {
       const bool end = tiles == nT;
       if constexpr (MIS) {
@@ -278,7 +271,7 @@ struct RowCopier
          // the ninth block, lane = row (the row may end in it also left of the strip's last tile)
          const uint32_t sh = (uint32_t)(uintptr_t)after & 15u;
          const int n = max(0, min(16, (nx + (end ? 0 : G::EL)) * B - 128 + (int)sh));
-         cpAsync<16>(dst + (uint32_t)(lane * G::PITCH + 128), after - sh - (n > 0 ? 0 : 128), n);
+         CP::template copy<16>(dst + (uint32_t)(lane * G::PITCH + 128), after - sh - (n > 0 ? 0 : 128), n);
          after -= tile;
       } else if (vec) {
          const char *q = p + (end ? adj : 0);
@@ -287,12 +280,12 @@ struct RowCopier
          if (wide) {
             const uint32_t step = 4u * (uint32_t)sy;
 #pragma unroll
-            for (int i = 0; i < 8; i++) { cpAsync<16>(d + (uint32_t)(i * 4 * G::PITCH), q + (uint64_t)(step * (uint32_t)i), n); }
+            for (int i = 0; i < 8; i++) { CP::template copy<16>(d + (uint32_t)(i * 4 * G::PITCH), q + (uint64_t)(step * (uint32_t)i), n); }
          } else {
             const int r0 = lane >> 3;
 #pragma unroll 1
             for (int i = 0; i < 8; i++) {
-               cpAsync<16>(d + (uint32_t)(i * 4 * G::PITCH), q + (int64_t)(min(r0 + 4 * i, last) - min(r0, last)) * sy, n);
+               CP::template copy<16>(d + (uint32_t)(i * 4 * G::PITCH), q + (int64_t)(min(r0 + 4 * i, last) - min(r0, last)) * sy, n);
             }
          }
       } else {
@@ -303,16 +296,16 @@ struct RowCopier
          if (wide) {
             const uint32_t step = (uint32_t)R * (uint32_t)sy;
 #pragma unroll 8
-            for (int i = 0; i < G::EL; i++) { cpAsync<B>(d + (uint32_t)(i * R * G::PITCH), p + (uint64_t)(step * (uint32_t)i), n); }
+            for (int i = 0; i < G::EL; i++) { CP::template copy<B>(d + (uint32_t)(i * R * G::PITCH), p + (uint64_t)(step * (uint32_t)i), n); }
          } else {
 #pragma unroll 1
             for (int i = 0; i < G::EL; i++) {
-               cpAsync<B>(d + (uint32_t)(i * R * G::PITCH), p + (int64_t)(min(r0 + R * i, last) - min(r0, last)) * sy, n);
+               CP::template copy<B>(d + (uint32_t)(i * R * G::PITCH), p + (int64_t)(min(r0 + R * i, last) - min(r0, last)) * sy, n);
             }
          }
       }
       if (end) {
-         if (!MIS) { cpAsync<B>(dst + (uint32_t)(lane * G::PITCH + 128), after, nAfter); }
+         if (!MIS) { CP::template copy<B>(dst + (uint32_t)(lane * G::PITCH + 128), after, nAfter); }
          p += step0;
       }
       p -= tile;

@@ -19,3 +19,17 @@ def test_arena_allocator(tmp_path):
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert "arena check ok" in r.stdout
+
+
+def test_copies_stay_inside_the_field(tmp_path):
+    """The kernels' copy addresses on fields of any strides and offset (copy_check.cu), on the host."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    exe = tmp_path / "copy_check"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O1", "--expt-relaxed-constexpr",
+                    "-I", os.path.join(REPO, "mkf_b200", "csrc"), "-I", os.path.join(REPO, "include"),
+                    os.path.join(REPO, "tests", "copy_check.cu"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "copy check ok" in r.stdout
