@@ -1,6 +1,6 @@
-// ballot.cu - fused counting kernel for one threshold on fields of middle size, and for a few of
-// one test on larger FP64 fields and the largest FP32 fields off 16-byte boundaries: map words packed
-// by warp votes from registers.
+// ballot.cu - fused counting kernel for one threshold on fields of middle size, and for a few of one test
+// (two of any) on strided, flat or narrow fields and part of those off 16-byte boundaries (useBallots): map
+// words packed by warp votes from registers.
 //
 // The other kernel for few thresholds (words.cuh) lets each lane pack its own row from a copy of the
 // tile in shared memory. That costs fewer instructions per threshold, but a FP64 tile row holds only
@@ -224,63 +224,99 @@ static bool innerTiles(const WordTask &a, int enc)
    return a.X >= 32 && a.Y >= 32 && syb > 0 && syb * 31 < (int64_t)1 << 32;
 }
 
+template <typename T, int MODE, int K>
+static int launchBallotK(const WordTask &a, int enc, cudaStream_t s)
+{
+   constexpr bool F32 = sizeof(T) == 4;
+   if (!innerTiles(a, enc)) { return launchBallotT<T, MODE, K, false, 2, false>(a, s); }
+   if constexpr (F32 && K <= 2) {
+      if (a.D >= kBlPfDepth) { return launchBallotT<T, MODE, K, true, 2, true>(a, s); }
+      return launchBallotT<T, MODE, K, true, 4, false>(a, s);
+   }
+   return launchBallotT<T, MODE, K, true, F32 ? 3 : 2, false>(a, s);
+}
+
 template <typename T, int MODE>
 static int launchBallotM(const WordTask &a, int enc, cudaStream_t s)
 {
-   constexpr bool F32 = sizeof(T) == 4;
-   if constexpr (!F32 && MODE < 3) {
-      if (a.K == 2) { return launchBallotT<T, MODE, 2, true, 2, false>(a, s); }
-      if (a.K == 3) { return launchBallotT<T, MODE, 3, true, 2, false>(a, s); }
-      if (a.K == 4) { return launchBallotT<T, MODE, 4, true, 2, false>(a, s); }
-      if (a.K == 5) { return launchBallotT<T, MODE, 5, true, 2, false>(a, s); }
+   if (a.K == 1) { return launchBallotK<T, MODE, 1>(a, enc, s); }
+   if (a.K == 2) { return launchBallotK<T, MODE, 2>(a, enc, s); }
+   if constexpr (MODE < 3) {
+      if (a.K == 3) { return launchBallotK<T, MODE, 3>(a, enc, s); }
+      if (a.K == 4) { return launchBallotK<T, MODE, 4>(a, enc, s); }
+      if (a.K == 5) { return launchBallotK<T, MODE, 5>(a, enc, s); }
+      if constexpr (sizeof(T) == 8) {
+         if (a.K == 6) { return launchBallotK<T, MODE, 6>(a, enc, s); }
+      }
    }
-   if constexpr (F32 && MODE < 3) {
-      if (a.K == 2 && a.D >= kBlPfDepth) { return launchBallotT<T, MODE, 2, true, 2, true>(a, s); }
-      if (a.K == 2) { return launchBallotT<T, MODE, 2, true, 4, false>(a, s); }
-      if (a.K == 3) { return launchBallotT<T, MODE, 3, true, 3, false>(a, s); }
-      if (a.K == 4) { return launchBallotT<T, MODE, 4, true, 3, false>(a, s); }
-      if (a.K == 5) { return launchBallotT<T, MODE, 5, true, 3, false>(a, s); }
-   }
-   if (!innerTiles(a, enc)) { return launchBallotT<T, MODE, 1, false, 2, false>(a, s); }
-   if (F32 && a.D >= kBlPfDepth) { return launchBallotT<T, MODE, 1, true, 2, F32>(a, s); }
-   return launchBallotT<T, MODE, 1, true, F32 ? 4 : 2, false>(a, s);
+   setError("vote kernel: %d thresholds", a.K);
+   return MKF_ERR_UNSUPPORTED;
 }
 
 template <typename T>
 static int dispatchBallot(const WordTask &a, int enc, cudaStream_t s)
 {
-   switch (a.mode[0]) {
+   switch (a.K == 2 && a.mode[1] != a.mode[0] ? 3 : a.mode[0]) {
       case 1: return launchBallotM<T, 1>(a, enc, s);
       case 2: return launchBallotM<T, 2>(a, enc, s);
       default: return launchBallotM<T, 3>(a, enc, s);
    }
 }
 
-// B200, device time of a call, this kernel against the other (words.cuh): FP32 64^3 7.9 / 6.9 us,
-// 128^3 8.3 / 8.9, 256^3 18.8 / 20.2, 301 x 333 x 277 33.7 / 34.6, 512^3 115 / 109,
-// 128 x 2048 x 2048 398 / 359; FP64 64^3 8.0 / 6.1, 128^3 9.2 / 9.6, 256 x 512 x 512 86 / 97,
-// 333 x 401 x 487 85 / 111. Four thresholds on larger FP64 fields: 256 x 512 x 512 plane waves 131 / 146,
-// GRF 158 / 161. Two to five on FP64 rows off 16-byte boundaries, where the other kernel's tile rows are
-// a ninth wider and fewer warps fit: 333 x 401 x 487 GRF, 3 thresholds 155 / 170, 4 158 / 181;
-// 301 x 333 x 277, 2 61 / 64, 3 82 / 79, 4 85 / 87; 100 x 101 x 99, 3 18 / 12.
-// The largest FP32 fields off 16-byte boundaries: this kernel gains where most tiles are uniform, and
-// the others' cost does not depend on the content (5: the rank table), 599 x 611 x 515, balls with noise: 2
-// thresholds 202 / 213, 3 241 / 293, 4 292 / 371, 5 347 / 387; plane waves 258 / 220, 340 / 311, 320 / 385, 402 /
-// 388; GRF 310 / 269, 427 / 378, 426 / 425, 527 / 391; 861 x 841 x 512 balls, 5 533 / 725; 478 x 768 x 993
-// GRF, 1 316 / 332. At 499 x 501 x 503 (below the line) balls 156 / 149, 185 / 193, 223 / 220, 269 / 268, GRF
-// 221 / 186, 319 / 257, 315 / 249, 381 / 271. The content is not known here; the line keeps the balls' worst
-// case.
+// Where this kernel counts a field. Its cost follows the content (uniform cells cost nothing), the others'
+// hardly does, and the content is not known here. So a line stands where this kernel is the faster one on
+// Gaussian fields (GRF), plane waves and balls with noise alike, or by more on some than slower on others.
+// B200, time of a call with the other kernel over that with this one, on GRF / waves / balls:
+//  one threshold, word kernel: FP32 64^3 0.87, 128^3 1.07, 256^3 1.07; aligned rows 512^3 0.95, 128 x 2048 x 2048
+//   0.90; other rows 500^3 1.04 / 1.02 / 1.17, 17 x 2048 x 2048 1.32 / 1.24 / 1.40, strided 500^3 1.9; FP64 64^3 0.76,
+//   128^3 1.04, 256 x 512 x 512 1.13, 333 x 401 x 487 1.31
+//  two to four, word kernel: 100^3 0.7, 128^3 0.9;
+//   strided x: FP32 128^3 0.9, 200 x 210 x 190 0.85 to 1.0, 256^3 1.1 to 1.3, 500^3 1.26 to 1.7; FP64 160 x 150 x 170 0.9
+//   to 1.07, 200 x 210 x 190 1.2 to 1.7; 512 x 6 x 512 FP32 1.3 to 1.5, 512 x 40 x 512 1.05 to 1.16, 512 x 512 x 20 1.1, FP64 1.25;
+//   few planes: 2 x 2048 x 2048 FP32 other rows 1.3, FP64 aligned 1.05 to 1.2, other rows 1.6 to 1.9; 9 x 1024 x 1024
+//   1.0 to 1.25, 1.0 to 1.25, 1.3 to 1.6; 5 x 1024 x 1024 FP64 aligned 2 thresholds 1.08 / 0.97 / 1.12, 4 0.98 / 0.93 / 0.85;
+//   33 x 1024 x 1024 FP32 other rows 1.1 / 0.95 / 1.2; 17 x 512 x 512 1.0 / 0.88 / 1.05, FP64 1.2 / 1.05 / 1.2;
+//   few columns: 512 x 512 x 20 other rows FP32 1.1 (2000 x 1000 x 17 0.9 / 0.93 / 1.08), FP64 1.2, aligned FP64 1.15; where the word kernel's tiles fit the row
+//   and the votes' 31 cells do not, FP64 512 x 512 x 8 4 thresholds 0.75, 2000 x 1000 x 17 0.6 to 0.8, FP32 512 x 512 x 33 0.7;
+//   few rows: 512 x 6 x 512 FP32 1.1, FP64 1.25 to 1.5; 512 x 40 x 512 FP64 1.03 to 1.15, other rows 1.1 to 1.3;
+//   2000 x 20 x 1000 FP64 aligned 4 thresholds 0.86 / 0.91 / 1.07;
+//   thick fields: FP32 other rows 400^3 2 and 3 thresholds 0.84 / 0.8 / 1.04, 4 1.0 / 1.12 / 1.22 (from 2^26 voxels
+//   on again 0.80 / 1.0 / 1.05, up to 2^27: 599 x 611 x 515 balls 3 thresholds 1.22, 4 1.27, 861 x 841 x 512 5 1.36);
+//   FP64 aligned 0.9 to 1.07 but 4 thresholds from 2^24 voxels on 0.97 / 1.06 / 1.07; other rows 2 thresholds
+//   200 x 210 x 190 0.99 / 1.09 / 1.18, 4 0.93 / 1.15 / 1.11, from 2^24 voxels on 1.07 to 1.2
+//  five and six, rank table: strided x FP32 300 x 333 x 277 0.94 / 1.07 / 1.10, 500^3 0.95 / 1.28 / 1.27, FP64 300 x 333 x
+//   277 1.15, 500^3 1.35, few rows (512 x 9 x 1024) 0.55; 2 x 2048 x 2048 1.2 to 1.3, 5 x 1024 x 1024 0.9 to 1.0, 9 x 4096
+//   x 4096 0.9 / 1.05 / 1.26; rows of less than 32 elements 1.4 to 2 (the staged kernel does not take them).
 bool useBallots(const WordTask &a, int enc)
 {
+   const bool f64 = enc == ENC_F64, aligned = wordRowsAligned(a, enc), strided = a.sx != 1;
    const double voxels = (double)a.X * a.Y * a.Z;
-   const bool largeF32 = enc == ENC_F32 && voxels >= (double)(1 << 27) && !wordRowsAligned(a, enc);
-   if (a.K == 1) { return voxels >= (double)(1 << 20) && (enc == ENC_F64 || voxels < (double)(1 << 26) || largeF32); }
-   if (!(enc == ENC_F64 || largeF32) || a.K > 5 || voxels < (double)(1 << 24) || !innerTiles(a, enc)) { return false; }
-   if (enc == ENC_F64 && a.K != 4 && wordRowsAligned(a, enc)) { return false; }
-   for (int k = 0; k < a.K; k++) {
+   if (a.K == 1) { return voxels >= (double)(1 << 20) && (f64 || !aligned || voxels < (double)(1 << 26)); }
+   if (a.K > (f64 ? 6 : 5) || voxels < (double)(a.Y < 9 ? 1 << 20 : 1 << 21)) { return false; }
+   for (int k = 0; k < a.K && a.K > 2; k++) {  // (two thresholds may differ in their tests)
       if (a.mode[k] != a.mode[0] || a.mode[k] == 3) { return false; }
    }
-   return true;
+   // cells that either kernel's tiles cover in a row
+   const int el = f64 ? 16 : 32, word = (a.X - 1 + el - 1) / el * el, vote = (a.X - 1 + 30) / 31 * 31;
+   const bool narrow = a.X < 64 && (f64 || voxels < (double)(1 << 24));
+   if (a.X < 64 && 10 * vote > 13 * word && !(f64 && strided && a.X >= 32)) { return false; }
+   if (a.K >= 5) {
+      if (a.X < 32) { return true; }
+      if (a.Y < 64) { return false; }
+      if (strided) { return voxels >= (double)(f64 ? 3 << 23 : 1 << 25) || (a.Z < 10 && voxels >= (double)(1 << 23)); }
+      if (a.Z < 8 && voxels >= (double)(1 << 23)) { return a.K == 5 ? f64 || !aligned : !aligned && a.Z < 5; }
+      return a.K == 5 && !f64 && !aligned && voxels >= (double)(1 << 27);
+   }
+   if (strided) { return narrow || a.Y < 64 || (a.Z < 10 && voxels >= (double)(1 << 23)) || voxels >= (double)(f64 ? 3 << 21 : 3 << 22); }
+   if (f64 && aligned) {
+      const bool large = voxels >= (double)(1 << 24);
+      return (a.X < 32 && a.K < 4) || (a.Y < 64 && (a.K < 4 || !large)) || (a.Z < 10 && voxels >= (double)(a.K == 2 ? 1 << 22 : 1 << 23)) ||
+             (a.K == 4 && large && innerTiles(a, enc));
+   }
+   if (f64) { return narrow || a.Y < 64 || a.Z < 34 || voxels >= (double)(a.K == 3 ? 1 << 24 : 1 << 22); }
+   if (aligned) { return a.Y < 9; }
+   if (narrow || a.Y < (a.K == 4 ? 64 : 16) || a.Z < (voxels < (double)(1 << 23) ? 10 : 34) || voxels >= (double)(1 << 27)) { return true; }
+   return a.K == 4 && voxels >= (double)(1 << 24) && voxels < (double)(1 << 26);
 }
 
 int launchBallots(WordTask &a, int enc, cudaStream_t s)
@@ -291,6 +327,12 @@ int launchBallots(WordTask &a, int enc, cudaStream_t s)
                     sizeDepth(kBlD, (long long)a.nStripX * a.nTileY, a.Z, (long long)smCount() * kBlItemsPerSM));
    a.nSlabZ = (a.Z - 1 + a.D - 1) / a.D;
    a.nItems = (long long)a.nStripX * a.nTileY * a.nSlabZ;
+   if (a.K == 2 && a.mode[1] != a.mode[0]) {  // both made "f > tlo or f < thi", the test not wanted never true
+      for (int k = 0; k < 2; k++) {
+         if (!(a.mode[k] & 1)) { a.tlo[k] = INFINITY; }
+         if (!(a.mode[k] & 2)) { a.thi[k] = -INFINITY; }
+      }
+   }
    return enc == ENC_F32 ? dispatchBallot<float>(a, enc, s) : dispatchBallot<double>(a, enc, s);
 }
 

@@ -171,13 +171,16 @@ int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, Fie
 
 int countVarying(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, cudaStream_t s)
 {
-   bool votes = false;  // five thresholds of a large FP32 field off 16-byte boundaries (useBallots)
-   if (q.cls >= 0 && q.n == 5 && pF->enc == ENC_F32) {
+   bool words = q.cls < 0 || q.n <= kWordThresholds;
+   if (!words && q.n <= (pF->enc == ENC_F32 ? 5 : 6)) {
+      // votes (useBallots), or a field of too few columns or rows for the staged rank-table kernel (5 thresholds,
+      // word kernel / rank table read from global memory, us: 64 x 64 x 20 FP32 17 / 24, FP64 14 / 24, 2000 x 1000 x 17
+      // FP64 78 / 200, 64 x 6 x 64 FP32 14 / 20; but 512 x 6 x 512 FP64 1.5 x)
       WordTask w;
       fillWordTask(w, pF, pT, q, 0, q.n, 0);
-      votes = useBallots(w, pF->enc);
+      words = useBallots(w, pF->enc) || w.X < 32 || (w.Y < 9 && (double)w.X * w.Y * w.Z < (double)(1 << 19));
    }
-   if (q.cls >= 0 && q.n > kWordThresholds && !votes) {
+   if (!words) {
       FusedArgs a;
       fillRankArgs(a, pF, pT, q, 0);
       a.out = out;

@@ -485,8 +485,11 @@ int launchThermo(FusedArgs &a, int enc, cudaStream_t s)
    a.lutC = prepareKeys(a, enc);
    if (a.lutC == 0) { return MKF_ERR_UNSUPPORTED; }
    const long long perPlane = (long long)((a.X - 1 + 30) / 31) * ((a.Y - 1 + THERMO_TY - 1) / THERMO_TY);
-   // up to 16 thresholds on fields of at least one tile: tiles staged in shared memory
-   if (thermoRingEligible(a)) {
+   // up to 16 thresholds on fields of at least one tile: tiles staged in shared memory; not so large FP64
+   // fields with strided x, whose elements are copied one by one (sx = 2, B200, us, staged / global memory: 256^3
+   // 12 thresholds 83 / 82, 300 x 333 x 277 8 1.13 x, 500^3 8 1.24 x, 16 1.14 to 1.22 x, 17 x 2048 x 2048 8 1.22 x)
+   const bool farColumns = enc == ENC_F64 && a.sx != 1 && (double)a.X * a.Y * a.Z >= (double)(3 << 23);
+   if (thermoRingEligible(a) && !farColumns) {
       const int family = thermoRingFamily(a, enc);
       itemGrid(a, tunedDepth(family, enc, a.K, a.X, a.Y, a.Z, ringDepth(perPlane, a.Z - 1, (long long)smCount() * kTmWarpsPerSM)));
       const int rc = launchThermoRing(a, enc, tunedVariant(family, enc, a.K, a.X, a.Y, a.Z, 0), s);

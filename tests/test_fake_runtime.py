@@ -244,3 +244,50 @@ for shape in ((64, 512, 1024), (128, 256, 512), (33, 700, 2048)):
         assert cost(W, warps) <= 1.0001 * cost(1, 16), (shape, depth, W)
         assert lib.mkfTuneSet(C.byref(d), C.byref(th.ts), 0, 0, None) == 0
 """)
+
+
+def test_kernel_of_a_call(fake):
+    """Which kernel counts a field, on both sides of each line of the routing."""
+    fake(r"""
+def kernel(dt, shape, kind, k, m=4):
+    Z, Y, X = shape
+    d = {"aligned": lambda: field(shape, dt, 0, (Y * (X + 3) // 4 * 4 * 1, (X + 3) // 4 * 4, 1)), "odd": lambda: field(shape, dt, 1, (Y * (X | 1), X | 1, 1)),
+         "strided": lambda: field(shape, dt, 0, (2 * Y * X, 2 * X, 2))}[kind]()
+    if kind == "aligned":
+        d = field(shape, dt, 0, (Y * ((X + 3) // 4 * 4), (X + 3) // 4 * 4, 1))
+    rc, names = count(d, k, m)
+    assert rc == 0
+    n = names[-1]
+    return "vote" if "ballot" in n else "word" if "wordBPFD" in n else "staged" if "thermoTma" in n else "global"
+
+F, D = np.float32, np.float64
+table = [
+    # one threshold
+    (F, (64, 127, 128), "aligned", 1, "word"), (F, (64, 129, 128), "aligned", 1, "vote"), (F, (128, 725, 728), "aligned", 1, "word"),
+    (F, (128, 725, 728), "odd", 1, "vote"), (F, (128, 725, 728), "strided", 1, "vote"), (D, (512, 512, 512), "aligned", 1, "vote"),
+    # thick fields
+    (F, (300, 300, 300), "aligned", 4, "word"), (F, (300, 300, 300), "odd", 3, "word"), (F, (300, 300, 300), "odd", 4, "vote"), (F, (200, 200, 200), "odd", 4, "word"),
+    (F, (500, 500, 500), "odd", 4, "word"), (F, (600, 600, 600), "odd", 3, "vote"), (F, (600, 600, 600), "odd", 5, "vote"),
+    (D, (300, 300, 300), "aligned", 3, "word"), (D, (300, 300, 300), "aligned", 4, "vote"), (D, (200, 200, 200), "aligned", 4, "word"),
+    (D, (200, 200, 200), "odd", 2, "vote"), (D, (200, 200, 200), "odd", 3, "word"), (D, (300, 300, 300), "odd", 3, "vote"),
+    # strided, flat, narrow
+    (F, (200, 200, 200), "strided", 3, "word"), (F, (250, 250, 250), "strided", 3, "vote"), (D, (160, 160, 160), "strided", 3, "word"),
+    (D, (200, 200, 200), "strided", 3, "vote"), (D, (200, 200, 200), "strided", 5, "staged"), (D, (300, 300, 300), "strided", 5, "vote"),
+    (F, (300, 300, 300), "strided", 5, "staged"), (F, (400, 400, 400), "strided", 5, "vote"), (F, (9000, 9, 1024), "strided", 5, "staged"),
+    (D, (300, 300, 300), "strided", 6, "vote"), (D, (200, 200, 200), "strided", 6, "staged"), (F, (300, 300, 300), "strided", 6, "staged"),
+    (D, (300, 300, 300), "strided", 8, "global"), (D, (256, 256, 256), "strided", 8, "staged"), (F, (300, 300, 300), "strided", 8, "staged"),
+    (F, (2, 2048, 2048), "odd", 2, "vote"), (F, (40, 512, 512), "odd", 2, "word"), (D, (9, 1024, 1024), "aligned", 2, "vote"), (D, (17, 1024, 1024), "aligned", 2, "word"),
+    (D, (2, 2048, 2048), "aligned", 5, "vote"), (D, (9, 2048, 2048), "aligned", 5, "staged"), (D, (2, 2048, 2048), "odd", 6, "vote"),
+    (F, (512, 6, 1024), "aligned", 2, "vote"), (F, (512, 10, 1024), "aligned", 2, "word"), (F, (512, 10, 1024), "odd", 2, "vote"),
+    (F, (17, 512, 512), "odd", 2, "word"), (F, (17, 1024, 1024), "odd", 2, "vote"), (D, (5, 1024, 1024), "aligned", 3, "word"),
+    (D, (2000, 1000, 17), "aligned", 3, "word"), (D, (2000, 1000, 20), "aligned", 3, "vote"), (F, (512, 512, 33), "odd", 2, "word"), (F, (512, 512, 40), "odd", 2, "vote"),
+    (D, (2000, 20, 1000), "aligned", 4, "word"), (D, (512, 40, 512), "aligned", 4, "vote"), (D, (512, 512, 17), "aligned", 6, "word"),
+    (F, (512, 512, 20), "odd", 5, "vote"), (D, (512, 512, 20), "aligned", 6, "vote"), (D, (512, 6, 512), "aligned", 5, "global"), (F, (512, 512, 20), "aligned", 6, "global"), (F, (64, 64, 20), "aligned", 5, "word"),
+    (D, (64, 6, 64), "aligned", 6, "word"),
+]
+for dt, shape, kind, k, want in table:
+    assert kernel(dt, shape, kind, k) == want, (dt, shape, kind, k, want, kernel(dt, shape, kind, k))
+# differing tests: two by votes, three by words
+assert kernel(D, (300, 300, 300), "odd", 2, [4, 1]) == "vote" and kernel(D, (300, 300, 300), "odd", 3, [4, 1, 4]) == "word"
+assert kernel(D, (300, 300, 300), "odd", 3, [4, 3, 4]) == "vote"  # (<= is > counted negated)
+""")
