@@ -26,7 +26,7 @@ struct FusedArgs
    double thi[64];       // sorted thresholds for the "f >= t" test, +inf padded
    // thermometer kernel: order-preserving 32-bit keys of the thresholds it compares against
    // (the high word for FP64 fields), sorted, and the most thresholds sharing one bucket of the
-   // 2^14-bucket rank table (1..4; 0 = the table cannot rank these thresholds)
+   // 2^14-bucket rank table
    uint32_t tkey[MKF_MAX_THRESH];
    int lutC;
 };

@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kThWarps * 32, THERMO_MINB) thermoBPFD(const _
 {
    __shared__ ThermoShared S;
    extern __shared__ uint32_t sHist[];
-   ctaSetup(a, S, sHist);
+   ctaSetup<false, (CMAX > 1)>(a, S, sHist);
    const long long gw = (long long)blockIdx.x * kThWarps + (threadIdx.x >> 5);
    const long long nw = (long long)gridDim.x * kThWarps;
    unsigned long long cells = 0;
@@ -333,7 +333,7 @@ static bool innerTiles(const P &a, int enc)
 }
 
 // Fill the key table of a thermometer pass and return the most thresholds sharing one bucket of
-// the rank table (1..4), or 0 when more share one (the word kernels count such passes).
+// the rank table.
 template <typename P>
 static int prepareKeys(P &a, int enc)
 {
@@ -344,7 +344,7 @@ static int prepareKeys(P &a, int enc)
       run = ((a.tkey[k] >> kLutShift) == (a.tkey[k - 1] >> kLutShift)) ? run + 1 : 1;
       most = std::max(most, run);
    }
-   return most <= 4 ? most : 0;
+   return most;
 }
 
 // Work-item grid of a field for the thermometer kernels (TY rows, D planes, 31 cells per item).
@@ -363,7 +363,7 @@ static void itemGrid(P &a, int D)
 bool prepareThermoTask(FieldTask &t, int enc, int depth)
 {
    t.lutC = prepareKeys(t, enc);
-   if (t.lutC == 0) { return false; }
+   if (t.lutC > kThCandidates) { return false; }
    t.variant = (enc == ENC_F32 ? 0 : 2) + (t.rankHi ? 1 : 0) + (innerTiles(t, enc) ? 4 : 0) + (t.lutC > 1 ? 8 : 0);
    itemGrid(t, depth > 0 ? depth : THERMO_D);
    return true;
@@ -483,7 +483,12 @@ static int ringDepth(long long perPlane, int cellsZ, long long warps)
 int launchThermo(FusedArgs &a, int enc, cudaStream_t s)
 {
    a.lutC = prepareKeys(a, enc);
-   if (a.lutC == 0) { return MKF_ERR_UNSUPPORTED; }
+   // Buckets of more thresholds than the kernel compares send their elements to the exact rank. The word kernel
+   // reads the field once for every 8 thresholds instead, which is faster but for many thresholds and larger
+   // fields (B200, us, word kernel / this, thresholds 4 / K around 300 on GRF): 400 x 388 x 416 FP32 17 616 / 729, 24
+   // 898 / 1004, 32 1205 / 1126, plane waves 24 758 / 742, 32 1021 / 810, FP64 24 1139 / 1025, 32 1528 / 1150;
+   // 2 x 2048 x 2048 FP64 24 169 / 134; 200 x 210 x 190 FP32 24 163 / 182, 32 217 / 216.
+   if (a.lutC > kThCandidates && (a.K < 24 || (double)a.X * a.Y * a.Z < (double)(1 << 23))) { return MKF_ERR_UNSUPPORTED; }
    const long long perPlane = (long long)((a.X - 1 + 30) / 31) * ((a.Y - 1 + THERMO_TY - 1) / THERMO_TY);
    // up to 16 thresholds on fields of at least one tile: tiles staged in shared memory; not so large FP64
    // fields with strided x, whose elements are copied one by one (sx = 2, B200, us, staged / global memory: 256^3

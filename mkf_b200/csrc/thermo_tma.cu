@@ -668,7 +668,7 @@ bool tmaRowsAligned(const FusedArgs &a, int enc)
 
 bool thermoRingEligible(const FusedArgs &a)
 {
-   return a.K > 2 && a.K <= kTmMaxK && a.X >= 32 && a.Y >= 9 && a.Z >= 2 && a.lutC >= 1;
+   return a.K > 2 && a.K <= kTmMaxK && a.X >= 32 && a.Y >= 9 && a.Z >= 2;
 }
 
 int thermoRingFamily(const FusedArgs &a, int enc)

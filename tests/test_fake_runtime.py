@@ -287,6 +287,10 @@ table = [
 ]
 for dt, shape, kind, k, want in table:
     assert kernel(dt, shape, kind, k) == want, (dt, shape, kind, k, want, kernel(dt, shape, kind, k))
+# thresholds that share a bucket of the rank table
+for shape, k, want in (((200, 200, 200), 32, "wordBPFD"), ((210, 210, 210), 23, "wordBPFD"), ((210, 210, 210), 24, "thermoBPFD"), ((210, 210, 210), 8, "wordBPFD")):
+    rc, names = count(field(shape, D), k, 4, [300.0 + 0.05 * i for i in range(k)])
+    assert rc == 0 and all(want in n for n in names), (shape, k, names)
 # differing tests: two by votes, three by words
 assert kernel(D, (300, 300, 300), "odd", 2, [4, 1]) == "vote" and kernel(D, (300, 300, 300), "odd", 3, [4, 1, 4]) == "word"
 assert kernel(D, (300, 300, 300), "odd", 3, [4, 3, 4]) == "vote"  # (<= is > counted negated)

@@ -75,3 +75,22 @@ def test_strided_fp64_on_both_sides_of_its_line(mkf, cuda):
             t = np.linspace(-1.0, 1.2, k)
             got = mkf.field_bpfd(f, t, m)
             assert torch.equal(got, torch.stack([plain_counts(f, v, m) for v in t])), (shape, k)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("shape", [(90, 300, 301), (100, 300, 301)])
+def test_thresholds_that_share_a_bucket(mkf, cuda, dtype, shape):
+    """17 to 32 thresholds of one relation in one bucket or two of the rank table, below and above 2^23
+    voxels, with elements on the thresholds and special values."""
+    import torch
+
+    f = make(shape, dtype, cuda)
+    f = f.contiguous()
+    for k, m in ((17, 4), (24, 6), (32, 1), (32, 3)):
+        t = np.float32(300.0) + np.linspace(-1.0, 1.2, k).astype(np.float32)
+        g = f + 300.0
+        g.view(-1)[11::97] = float(t[k // 2])
+        got = mkf.field_bpfd(g, t, m)
+        for i in (0, 1, k // 2, k - 1):
+            assert torch.equal(got[i], plain_counts(g, float(t[i]), m)), (k, m, i)
+        assert torch.equal(got, torch.cat([mkf.field_bpfd(g, [float(v)], m) for v in t]))
