@@ -199,6 +199,7 @@ static int createPlan(MKFBatchPlan **pp, uint64_t *pBPFD, const MKFFieldDesc *pF
    std::vector<WordTask> wtasks[2];
    std::vector<BatchChunk> wchunks[2];
    size_t row = 0;
+   BatchMix mix;
    for (int i = 0; i < nF; i++) {
       const MKFFieldDesc *d = pF + i;
       const MKFThreshSet *ts = pT + i;
@@ -208,12 +209,17 @@ static int createPlan(MKFBatchPlan **pp, uint64_t *pBPFD, const MKFFieldDesc *pF
          freePlan(p);
          return MKF_ERR_ARG;
       }
+      mix.add(d, ts);
+   }
+   for (int i = 0; i < nF; i++) {
+      const MKFFieldDesc *d = pF + i;
+      const MKFThreshSet *ts = pT + i;
       const unsigned long long cells = (unsigned long long)(d->def[0] - 1) * (d->def[1] - 1) * (d->def[2] - 1);
       const size_t c0 = p->consts.size();
       FieldTask t;
       WordTask w;
       bool varying = false;
-      const int kind = planBatchField(d, ts, (int)row, t, w, p->consts, varying, depth);
+      const int kind = planBatchField(d, ts, (int)row, t, w, p->consts, varying, mix.wordMax(d->enc, depth), depth);
       for (size_t c = c0; c < p->consts.size(); c++) { p->constCells.push_back(cells); }
       if (cells > 0 && kind == kPlanWords) {
          const int e = d->enc == ENC_F32 ? 0 : 1;

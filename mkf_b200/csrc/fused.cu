@@ -122,18 +122,51 @@ void fillWordTask(WordTask &w, const MKFFieldDesc *pF, const MKFThreshSet *pT, c
    }
 }
 
-// Split one field of a batch (rows from row0): one or two varying thresholds, or up to kWordMaxK of
-// any relations, fill `w` for the batched word kernel (returns kPlanWords); more thresholds that share
-// one thermometer relation and fit the rank table fill `t` for the batched thermometer kernel
-// (kPlanThermo). Fields of kSoloVoxels or more with more than two thresholds fill the GPU on their
-// own, and the single-field kernels (specialised on the number of thresholds; the TMA-staged rank table
-// on aligned rows) count them faster: those fields, and the rest, take the single-field path
-// (kPlanSingle). A served burst of 64 fields of 32^3 to 320^3 with 1-8 thresholds: word kernel up to 2
-// thresholds 1902 us, up to 8 1750; the cut at 2^24 voxels instead of 2^23 1800, at 2^26 2015. Constant
-// maps are added to `consts`.
+// Fields of kSoloVoxels or more with more than two thresholds fill the GPU on their own, and the
+// single-field kernels (specialised on the number of thresholds; the TMA-staged rank table on aligned rows)
+// count them faster than the batched ones. A served burst of 64 fields of 32^3 to 320^3 with 1-8 thresholds:
+// the cut at 2^23 voxels 1750 us, at 2^24 1800, at 2^26 2015.
 static constexpr double kSoloVoxels = (double)(1 << 23);
+
+void BatchMix::add(const MKFFieldDesc *pF, const MKFThreshSet *pT)
+{
+   const int e = pF->enc == ENC_F32 ? 0 : 1;
+   const double vox = (double)pF->def[0] * (double)pF->def[1] * (double)pF->def[2];
+   ThreshSplit q;
+   splitThresholds(pT, q);
+   if (q.n == 0 || (q.n > 2 && (vox >= kSoloVoxels || q.n > kWordMaxK))) { return; }
+   if (q.n <= 2 || q.cls < 0) { words[e] = true; }
+   else {
+      fields[e]++;
+      voxels[e] += vox;
+      thresholds[e] += vox * q.n;
+   }
+}
+
+// A batch whose fields differ goes to the batched word kernel in one launch (fields of 1 to 8 thresholds,
+// 64 fields served: up to 2 thresholds in the word kernel and the rest in the rank table's 1869 us, all
+// 1537; plans of 40 to 70 fields 535 / 453, 774 / 607, 669 / 599). Where no field needs the word kernel the
+// rank table alone counts it, whose cost hardly grows with the thresholds. Word kernel over rank table, plans
+// (GRF / waves / balls): 400 fields of 12^3 to 20^3 3 thresholds 1.8, 8 2.9; 100 of 40^3 to 80^3 FP32 3 1.15, 5 1.25,
+// 8 1.65; 64 of 60^3 to 120^3 FP32 3 1.02 / 0.86 / 0.86, 4 1.1 / 1.0 / 1.04, 5 1.26 / 1.14 / 1.25, FP64 3 1.14 / 1.03 / 1.08;
+// 24 of 150^3 to 200^3 FP32 3 1.0 / 0.76 / 0.71, 4 1.05 / 0.9 / 0.87, 5 1.16 / 1.0 / 0.97, FP64 3 1.08 / 0.94 / 0.87, 4 1.13 /
+// 1.05 / 1.0; in one-shot batches (shallow items, time with the host's) 0.9 to 0.95 up to 5 thresholds, from 100^3 on 6
+// 1.0 to 1.2, 8 1.1 to 1.4.
+int BatchMix::wordMax(int enc, int depth) const
+{
+   const int e = enc == ENC_F32 ? 0 : 1;
+   if (words[e] || fields[e] == 0) { return kWordMaxK; }
+   const double vox = voxels[e] / fields[e], k = thresholds[e] / voxels[e];
+   const bool rank = depth < 0 ? vox >= (double)(1 << 20) && k >= 5.5 : vox < (double)(e ? 1 << 20 : 1 << 19) || k >= (e ? 3.5 : 4.5);
+   return rank ? 2 : kWordMaxK;
+}
+
+// Split one field of a batch (rows from row0): up to kWordMaxK thresholds of any relations, but of one
+// relation up to wordMax (BatchMix), fill `w` for the batched word kernel (returns kPlanWords); more
+// thresholds that share one thermometer relation and fit the rank table fill `t` for the batched thermometer
+// kernel (kPlanThermo); the rest takes the single-field path (kPlanSingle). Constant maps are added to `consts`.
 int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, FieldTask &t, WordTask &w,
-                   std::vector<ConstEntry> &consts, bool &anyVarying, int depth)
+                   std::vector<ConstEntry> &consts, bool &anyVarying, int wordMax, int depth)
 {
    memset(&t, 0, sizeof(t));
    memset(&w, 0, sizeof(w));
@@ -148,11 +181,13 @@ int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, Fie
    for (int c = 0; c < q.nConst; c++) { consts.push_back({row0 + q.constIdx[c], q.constBin[c]}); }
    anyVarying = q.n > 0;
    if (q.n == 0) { return kPlanSingle; }
-   if (q.n <= 2 || (q.n <= kWordMaxK && vox < kSoloVoxels)) {
+   const bool word = q.n <= 2 || (q.n <= kWordMaxK && vox < kSoloVoxels);
+   auto words = [&]() {
       fillWordTask(w, pF, pT, q, 0, q.n, row0);
       fillWordGrid(w, pF->enc, depth > 0 ? depth : 32, q.n <= 4 ? 2 : 1);
       return kPlanWords;
-   }
+   };
+   if (word && (q.cls < 0 || q.n <= wordMax)) { return words(); }
    if (q.cls < 0 || vox >= kSoloVoxels) { return kPlanSingle; }
    FusedArgs a;
    fillRankArgs(a, pF, pT, q, row0);
@@ -166,7 +201,8 @@ int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, Fie
    t.rankHi = a.rankHi;
    t.complement = a.complement;
    t.nanRank = a.nanRank;
-   return prepareThermoTask(t, pF->enc, depth) ? kPlanThermo : kPlanSingle;
+   if (prepareThermoTask(t, pF->enc, depth)) { return kPlanThermo; }
+   return word ? words() : kPlanSingle;
 }
 
 int countVarying(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, const ThreshSplit &q, cudaStream_t s)

@@ -140,9 +140,18 @@ void floatBoundsPlain(double t, double &tlo, double &thi);
 int fieldBPFD(uint64_t *out, const MKFFieldDesc *pF, const MKFThreshSet *pT, int flags, cudaStream_t s);
 
 enum { kPlanSingle = 0, kPlanThermo = 1, kPlanWords = 2 };
+// The fields of a batch that either batched kernel could count, by element type, and which of them does.
+struct BatchMix
+{
+   bool words[2] = {false, false};  // some field needs the word kernel: 1 or 2 thresholds, or relations that differ
+   int fields[2] = {0, 0};          // the others of up to kWordMaxK thresholds: their number,
+   double voxels[2] = {0.0, 0.0}, thresholds[2] = {0.0, 0.0};  // voxels, and thresholds times voxels
+   void add(const MKFFieldDesc *pF, const MKFThreshSet *pT);
+   int wordMax(int enc, int depth) const;  // most thresholds of one relation for the word kernel
+};
 // depth: planes of cells per work item; 0 = each kernel's default, -1 = chosen by field size.
 int planBatchField(const MKFFieldDesc *pF, const MKFThreshSet *pT, int row0, FieldTask &t, WordTask &w,
-                   std::vector<ConstEntry> &consts, bool &anyVarying, int depth = 0);
+                   std::vector<ConstEntry> &consts, bool &anyVarying, int wordMax, int depth);
 
 // Slab depth (planes of cells per work item) of a single-field launch of kernel family `family`
 // (tune.cu): the depth mkfTune measured best for this kind of field, else `def`. A family is one kernel

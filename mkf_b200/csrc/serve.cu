@@ -168,17 +168,26 @@ static int issueLaunch(MKFServer *s, LaunchSlot &sl)
    std::vector<Const> consts;
    struct Single { Request *r; MKFFieldDesc d; };
    std::vector<Single> singles;
+   auto threshOf = [](const Request *r) {
+      MKFThreshSet ts;
+      ts.nT = (int32_t)r->t.size();
+      ts.mAll = r->mAll;
+      ts.t = r->t.data();
+      ts.m = r->m.empty() ? nullptr : r->m.data();
+      return ts;
+   };
+   BatchMix mix;
+   for (const Request *r : sl.reqs) {
+      const MKFThreshSet ts = threshOf(r);
+      mix.add(&r->field, &ts);
+   }
    for (Request *r : sl.reqs) {
       MKFFieldDesc d = r->field;
       if (r->staged) {
          d.p = r->staged;
          d.stride[0] = d.stride[1] = d.stride[2] = 0;
       }
-      MKFThreshSet ts;
-      ts.nT = (int32_t)r->t.size();
-      ts.mAll = r->mAll;
-      ts.t = r->t.data();
-      ts.m = r->m.empty() ? nullptr : r->m.data();
+      const MKFThreshSet ts = threshOf(r);
       clears.push_back({r->dCounts, (long long)ts.nT * 256});
       const unsigned long long cells =
          (unsigned long long)(d.def[0] - 1) * (unsigned long long)(d.def[1] - 1) * (unsigned long long)(d.def[2] - 1);
@@ -186,7 +195,7 @@ static int issueLaunch(MKFServer *s, LaunchSlot &sl)
       WordTask w;
       std::vector<ConstEntry> ce;
       bool varying = false;
-      const int kind = planBatchField(&d, &ts, 0, t, w, ce, varying, -1);  // depth by field size
+      const int kind = planBatchField(&d, &ts, 0, t, w, ce, varying, mix.wordMax(d.enc, -1), -1);  // depth by field size
       if (cells == 0) { continue; }
       if (kind == kPlanSingle && varying) {
          singles.push_back({r, d});  // counts every threshold, constant maps included
@@ -259,11 +268,7 @@ static int issueLaunch(MKFServer *s, LaunchSlot &sl)
    }
    for (size_t i = 0; i < singles.size() && rc == MKF_OK; i++) {
       Request *r = singles[i].r;
-      MKFThreshSet ts;
-      ts.nT = (int32_t)r->t.size();
-      ts.mAll = r->mAll;
-      ts.t = r->t.data();
-      ts.m = r->m.empty() ? nullptr : r->m.data();
+      const MKFThreshSet ts = threshOf(r);
       rc = fieldBPFD(r->dCounts, &singles[i].d, &ts, MKF_F_ACCUMULATE, st);
    }
    if (rc != MKF_OK) { return rc; }

@@ -295,3 +295,39 @@ for shape, k, want in (((200, 200, 200), 32, "wordBPFD"), ((210, 210, 210), 23, 
 assert kernel(D, (300, 300, 300), "odd", 2, [4, 1]) == "vote" and kernel(D, (300, 300, 300), "odd", 3, [4, 1, 4]) == "word"
 assert kernel(D, (300, 300, 300), "odd", 3, [4, 3, 4]) == "vote"  # (<= is > counted negated)
 """)
+
+
+def test_kernel_of_a_batch(fake):
+    """The batched rank table takes a batch none of whose fields needs the word kernel, if it is the faster
+    one for its sizes and thresholds; any other batch of up to 8 thresholds is one word kernel launch."""
+    fake(r"""
+def batch(dt, shapes, ks, plan, masks=None):
+    sets = [M._Thresholds(list(np.linspace(-1, 1, k)), 4 if masks is None else masks[i]) for i, k in enumerate(ks)]
+    n = len(sets)
+    descs = (_lib.MKFFieldDesc * n)(*[field(s, dt) for s in shapes])
+    ts = (_lib.MKFThreshSet * n)(*[s.ts for s in sets])
+    out = np.zeros((sum(ks), 256), np.uint64)
+    launches()
+    if plan:
+        h = C.c_void_p()
+        assert lib.mkfBatchPlanCreate(C.byref(h), out.ctypes.data, descs, ts, n) == 0
+        launches()
+        assert lib.mkfBatchPlanLaunch(h, None) == 0
+        names = [l[1] for l in launches()]
+        assert lib.mkfBatchPlanDestroy(h) == 0
+    else:
+        assert lib.mkfBatchBPFD(out.ctypes.data, descs, ts, n, 0, None) == 0
+        names = [l[1] for l in launches()]
+    assert all("wordBatch" in x or "thermoBatch" in x for x in names), names
+    return "".join(sorted({"w" if "wordBatch" in x else "r" for x in names}))
+
+F, D = np.float32, np.float64
+S = lambda n: [(n, n, n)] * 4
+for dt, n, k, plan, want in ((F, 16, 3, True, "r"), (F, 60, 8, True, "r"), (F, 90, 4, True, "w"), (F, 90, 5, True, "r"), (F, 150, 3, True, "w"), (F, 150, 8, True, "r"),
+                             (D, 90, 3, True, "r"), (D, 110, 3, True, "w"), (D, 110, 4, True, "r"), (F, 16, 8, False, "w"), (F, 90, 8, False, "w"),
+                             (F, 110, 5, False, "w"), (F, 110, 6, False, "r"), (D, 110, 8, False, "r"), (F, 16, 2, True, "w"), (F, 16, 12, False, "r")):
+    assert batch(dt, S(n), [k] * 4, plan) == want, (dt, n, k, plan)
+for plan in (True, False):
+    assert batch(F, S(150), [8, 8, 8, 1], plan) == "w" and batch(F, S(150), [8, 8, 8, 3], plan, [4, 4, 4, [4, 1, 2]]) == "w"
+    assert batch(F, S(150), [8, 8, 8, 12], plan) == "r" and batch(F, S(150), [1, 8, 8, 12], plan) == "rw"
+""")

@@ -94,3 +94,21 @@ def test_thresholds_that_share_a_bucket(mkf, cuda, dtype, shape):
         for i in (0, 1, k // 2, k - 1):
             assert torch.equal(got[i], plain_counts(g, float(t[i]), m)), (k, m, i)
         assert torch.equal(got, torch.cat([mkf.field_bpfd(g, [float(v)], m) for v in t]))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("n", [14, 93, 127])
+def test_batches_of_one_threshold_count(mkf, cuda, dtype, n):
+    """Batches by either batched kernel (3 to 8 thresholds for every field, and with one field that differs),
+    as a plan and in one shot, against the fields one at a time."""
+    import torch
+
+    fs = [make((n, n + i, n - i), dtype, cuda, 1, i) for i in range(3)]
+    for k, m in ((3, 4), (5, 6), (6, 1), (8, 3)):
+        for t in (np.linspace(-1.0, 1.2, k), 300.0 + 0.01 * np.arange(k)):  # (the second share a bucket)
+            for ks, ms in (([t] * 3, [m] * 3), ([t, t[:1], t], [m, 2, m])):
+                want = torch.cat([mkf.field_bpfd(f, v, w) for f, v, w in zip(fs, ks, ms)])
+                p = mkf.BatchPlan(fs, ks, ms)
+                assert torch.equal(p.launch(), want), (k, m)
+                p.close()
+                assert torch.equal(mkf.batch_bpfd(fs, ks, ms), want), (k, m)
