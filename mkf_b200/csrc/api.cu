@@ -258,7 +258,7 @@ static int createPlan(MKFBatchPlan **pp, uint64_t *pBPFD, const MKFFieldDesc *pF
    }
    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
       if (wtasks[k].empty()) { continue; }
-      wchunks[k] = wordChunks(wtasks[k]);
+      wchunks[k] = wordChunks(wtasks[k], k == 0 ? ENC_F32 : ENC_F64);
       e = cudaMalloc(&p->dWTasks[k], wtasks[k].size() * sizeof(WordTask));
       if (e == cudaSuccess) { e = cudaMalloc(&p->dWChunks[k], wchunks[k].size() * sizeof(BatchChunk)); }
       if (e == cudaSuccess) { e = cudaMemcpy(p->dWTasks[k], wtasks[k].data(), wtasks[k].size() * sizeof(WordTask), cudaMemcpyHostToDevice); }

@@ -83,11 +83,11 @@ struct BatchChunk
 
 // Cut a batch's fields (tasks of one kernel) into chunks. A CTA waits for its slowest warp at the end
 // of a chunk and fills its copy pipeline anew at the start, so chunks are as long as leaves every one
-// of `ctas` CTAs about four of them, in multiples of its warps, and the costliest come first: with
-// chunks of 64 items, 64 served fields gave 29 and 65 chunks to 148 SMs (733 and 638 us). cost: of an
-// item of a task.
-template <typename TASK, typename COST>
-std::vector<BatchChunk> cutChunks(const std::vector<TASK> &tasks, int ctas, int warps, int maxItems, COST cost)
+// of `ctas` CTAs about four of them, in multiples of the warps that count it, and the costliest come first:
+// with chunks of 64 items, 64 served fields gave 29 and 65 chunks to 148 SMs (733 and 638 us). cost: of an
+// item of a task; warps: of a CTA that count items of a task; at most maxRounds items each.
+template <typename TASK, typename COST, typename WARPS>
+std::vector<BatchChunk> cutChunks(const std::vector<TASK> &tasks, int ctas, int maxRounds, COST cost, WARPS warpsOf)
 {
    double total = 0.0;
    for (const TASK &t : tasks) { total += (double)t.nItems * cost(t); }
@@ -97,8 +97,9 @@ std::vector<BatchChunk> cutChunks(const std::vector<TASK> &tasks, int ctas, int 
    std::vector<BatchChunk> chunks;
    for (const auto &o : order) {
       const TASK &t = tasks[o.second];
-      long long n = (long long)(total / (4.0 * ctas) / -o.first / warps + 0.5) * warps;
-      n = n < warps ? warps : (n > maxItems ? maxItems : n);
+      const int warps = warpsOf(t);
+      long long n = (long long)(total / (4.0 * ctas) / -o.first / warps + 0.5);
+      n = (n < 1 ? 1 : n > maxRounds ? maxRounds : n) * warps;
       for (long long b = 0; b < t.nItems; b += n) { chunks.push_back({o.second, 0, b, b + n < t.nItems ? b + n : t.nItems}); }
    }
    return chunks;
@@ -209,7 +210,7 @@ bool useBallots(const WordTask &a, int enc);
 int launchWordsMoments(WordTask &a, int enc, cudaStream_t s);
 
 // Chunks of the batched kernels' tasks (words_batch.cu, thermo.cu).
-std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks);
+std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks, int enc);
 std::vector<BatchChunk> thermoChunks(const std::vector<FieldTask> &tasks);
 // The batched word kernel over the chunks of tasks of one element type (words_batch.cu).
 int launchWordsBatch(const WordBatchArgs &b, int enc, cudaStream_t s);

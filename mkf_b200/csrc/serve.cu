@@ -214,7 +214,7 @@ static int issueLaunch(MKFServer *s, LaunchSlot &sl)
    }
    std::vector<ThermoGroup> groups[2];  // thermometer chunks sorted into one run per kernel variant
    for (int k = 0; k < 2; k++) {
-      wchunks[k] = wordChunks(wtasks[k]);
+      wchunks[k] = wordChunks(wtasks[k], k == 0 ? ENC_F32 : ENC_F64);
       chunks[k] = thermoChunks(tasks[k]);
       if (!chunks[k].empty()) { groups[k] = groupThermoChunks(chunks[k], tasks[k]); }
    }

@@ -371,7 +371,7 @@ bool prepareThermoTask(FieldTask &t, int enc, int depth)
 
 std::vector<BatchChunk> thermoChunks(const std::vector<FieldTask> &tasks) 
 {
-   return cutChunks(tasks, 3 * smCount(), kThWarps, 8 * kThWarps, [](const FieldTask &t) { return t.D + 1.0; });
+   return cutChunks(tasks, 3 * smCount(), 8, [](const FieldTask &t) { return t.D + 1.0; }, [](const FieldTask &) { return kThWarps; });
 }
 
 std::vector<ThermoGroup> groupThermoChunks(std::vector<BatchChunk> &chunks, const std::vector<FieldTask> &tasks)

@@ -67,6 +67,13 @@ __host__ __device__ constexpr int wordWarpBytes(int nr, int K, int W, bool mis)
 // Dynamic shared memory of a CTA: 227 KB less the static part (histograms, a batch's task).
 constexpr int kWdDynBytes = 232448 - 1024 * (kWordMaxK + 1) - 2048;
 
+// Warps of a batch CTA that the memory holds for a field (its form for fields with unit x stride has larger
+// tiles: 14 of FP32, one threshold, 11 with eight).
+__host__ __device__ constexpr int wordBatchWarps(int nr, int K, int W, bool mis)
+{
+   return kWdDynBytes / wordWarpBytes(nr, K, W, mis) < kWdWarps ? kWdDynBytes / wordWarpBytes(nr, K, W, mis) : kWdWarps;
+}
+
 // A threshold as the map step uses it.
 struct alignas(16) RowThresh
 {

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(kWdWarps * 32, 1) wordBatch(const __grid_const
       const bool mis = F.sx == 1;
       const int bytes = wordWarpBytes(RowGeom<T, true>::NR, F.K, F.W, mis);
       const auto item = [&](int j) { return ch.begin + j; };
-      if (warp < kWdDynBytes / bytes) {
+      if (warp < wordBatchWarps(RowGeom<T, true>::NR, F.K, F.W, mis)) {
          if (!mis) { rowItems<T, false, 0, false>(F, item, ch.end, mem + (uint32_t)(warp * bytes), S); }
          else if (F.K == 1) { rowItems<T, false, 1, true>(F, item, ch.end, mem + (uint32_t)(warp * bytes), S); }
          else { rowItems<T, false, 0, true>(F, item, ch.end, mem + (uint32_t)(warp * bytes), S); }
@@ -52,10 +52,11 @@ __global__ void __launch_bounds__(kWdWarps * 32, 1) wordBatch(const __grid_const
    if (cur >= 0) { rowFlush(F, S); }
 }
 
-std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks) 
+std::vector<BatchChunk> wordChunks(const std::vector<WordTask> &tasks, int enc)
 {
    // tiles of an item, each about half a threshold's work before the thresholds'
-   return cutChunks(tasks, smCount(), kWdWarps, 16 * kWdWarps, [](const WordTask &t) { return (t.D + 1.0) * t.W * (t.K + 0.5); });
+   return cutChunks(tasks, smCount(), 16, [](const WordTask &t) { return (t.D + 1.0) * t.W * (t.K + 0.5); },
+                    [enc](const WordTask &t) { return wordBatchWarps(enc == ENC_F32 ? 4 : 2, t.K, t.W, t.sx == 1); });
 }
 
 template <typename T>

@@ -69,9 +69,13 @@ static size_t limitOf(const void *f)
    auto it = smemLimit.find({curDev, f});
    return it == smemLimit.end() ? 48 * 1024 : it->second;
 }
-Err cudaLaunchKernel(const void *f, Dim3 g, Dim3 b, void **, size_t smem, void *)
+// The first argument of the last batch kernel launched (tasks, chunks, number of chunks, counter).
+static unsigned char batchArgs[32];
+const void *fake_batch_args() { return batchArgs; }
+Err cudaLaunchKernel(const void *f, Dim3 g, Dim3 b, void **args, size_t smem, void *)
 {
    std::lock_guard<std::mutex> lk(mu);
+   if (kernelName[f].find("Batch") != std::string::npos) { memcpy(batchArgs, args[0], sizeof(batchArgs)); }
    if (smem > limitOf(f) || g.x == 0 || b.x == 0 || b.x > 1024) { return fail(BAD_VALUE); }
    launches.push_back(std::to_string(curDev) + " " + kernelName[f] + " " + std::to_string(smem) + " " +
                       std::to_string(g.x) + " " + std::to_string(b.x));

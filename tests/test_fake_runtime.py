@@ -331,3 +331,41 @@ for plan in (True, False):
     assert batch(F, S(150), [8, 8, 8, 1], plan) == "w" and batch(F, S(150), [8, 8, 8, 3], plan, [4, 4, 4, [4, 1, 2]]) == "w"
     assert batch(F, S(150), [8, 8, 8, 12], plan) == "r" and batch(F, S(150), [1, 8, 8, 12], plan) == "rw"
 """)
+
+
+def test_chunks_of_a_batch(fake):
+    """The chunks of a word kernel batch cover every item once, and each is a whole number of rounds of the
+    warps that count it, but for the last of a field."""
+    fake(r"""
+class Args(C.Structure):
+    _fields_ = [("tasks", C.c_void_p), ("chunks", C.c_void_p), ("n", C.c_int), ("counter", C.c_void_p)]
+class Chunk(C.Structure):
+    _fields_ = [("field", C.c_int), ("pad", C.c_int), ("begin", C.c_longlong), ("end", C.c_longlong)]
+
+fake.fake_batch_args.restype = C.POINTER(Args)
+for dt, nr in ((np.float32, 4), (np.float64, 2)):
+    for strides in (None, (2 * 90 * 90, 2 * 90, 2)):
+        for k in (1, 2, 5, 8):
+            masks = [4, 1] * k
+            sets = [M._Thresholds(list(np.linspace(-1, 1, k)), masks[:k]) for _ in range(40)]
+            descs = (_lib.MKFFieldDesc * 40)(*[field((90 - i, 90, 90), dt, 0, strides) for i in range(40)])
+            ts = (_lib.MKFThreshSet * 40)(*[s.ts for s in sets])
+            out = np.zeros((40 * k, 256), np.uint64)
+            h = C.c_void_p()
+            lib.mkfSetTuning(0)
+            assert lib.mkfBatchPlanCreate(C.byref(h), out.ctypes.data, descs, ts, 40) == 0
+            assert lib.mkfBatchPlanLaunch(h, None) == 0
+            assert any("wordBatch" in l[1] for l in launches())
+            a = fake.fake_batch_args().contents
+            chunks = list((Chunk * a.n).from_address(a.chunks))
+            mis = strides is None
+            W = 2 if k <= 4 else 1
+            warp = 2 * 32 * (176 if mis else 144) + 9 * 288 + k * (W * (nr // 2) + 3) * 128
+            warps = min(16, (232448 - 1024 * 9 - 2048) // warp)
+            for f in range(40):
+                mine = sorted((c.begin, c.end) for c in chunks if c.field == f)
+                assert mine[0][0] == 0 and all(p[1] == q[0] for p, q in zip(mine, mine[1:])), mine
+                assert all((e - b) % warps == 0 for b, e in mine[:-1]) and mine[-1][1] > mine[-1][0], (dt, k, warps, mine)
+            assert max(c.end - c.begin for c in chunks) > 0
+            assert lib.mkfBatchPlanDestroy(h) == 0
+""")
