@@ -4,21 +4,12 @@
 #include <mutex>
 #include <vector>
 #include "fused.cuh"
+#include "groups.cuh"
 
 namespace mkf {
 void measures(double r[4], const uint64_t h[256]);
-extern const uint8_t kGroupOf[256];
-extern const int kWK[22];
-extern const double kWS[22];
-extern const double kWM[22];
 
-// Device copy of the group weights and of the patterns sorted by group: group q holds patterns
-// cMember[cFirst[q]] .. cMember[cFirst[q + 1] - 1].
-__constant__ uint8_t cMember[256];
-__constant__ int cFirst[23];
-__constant__ int cWK[22];
-__constant__ double cWS[22];
-__constant__ double cWM[22];
+__constant__ GroupTables cGroups = groupTables();
 
 // One CTA per distribution, same arithmetic and order as measures() on the host, so the device and
 // host results are identical: the group sums are integers (any order), one thread each for the 22
@@ -36,7 +27,7 @@ __global__ void __launch_bounds__(128) measuresKernel(double *r, const uint64_t 
       uint64_t v = 0;
       if (t < 22) {
          uint64_t s = 0;
-         for (int q = cFirst[t]; q < cFirst[t + 1]; q++) { s += p[cMember[q]]; }
+         for (int q = cGroups.first[t]; q < cGroups.first[t + 1]; q++) { s += p[cGroups.member[q]]; }
          g[t] = s;
       } else if (t >= 96) {
          const int l = t - 96;
@@ -46,7 +37,7 @@ __global__ void __launch_bounds__(128) measuresKernel(double *r, const uint64_t 
       __syncthreads();
       // separate multiply and add (no fused multiply-add), as the host computes it
       if (t == 0 || t == 32) {
-         const double *w = t == 0 ? cWS : cWM;
+         const double *w = t == 0 ? cGroups.wS : cGroups.wM;
          double s = __dmul_rn((double)g[0], w[0]);
 #pragma unroll
          for (int q = 1; q < 22; q++) { s = __dadd_rn(s, __dmul_rn((double)g[q], w[q])); }
@@ -54,45 +45,13 @@ __global__ void __launch_bounds__(128) measuresKernel(double *r, const uint64_t 
       } else if (t == 64) {
          long long k = 0;
 #pragma unroll
-         for (int q = 0; q < 22; q++) { k += (long long)cWK[q] * (long long)g[q]; }
+         for (int q = 0; q < 22; q++) { k += (long long)cGroups.wK[q] * (long long)g[q]; }
          r[4 * i + 3] = (double)k / 24.0;
       } else if (t == 96) {
          r[4 * i + 0] = (double)v;
       }
       __syncthreads();
    }
-}
-
-// __constant__ memory belongs to each device: upload the tables once per device, on first use
-// with that device current.
-static std::mutex gConstMu;
-static bool gConstDone[64] = {};
-
-static int uploadConstants()
-{
-   int dev = 0;
-   cudaError_t e = cudaGetDevice(&dev);
-   if (e != cudaSuccess) { return cudaFail(e, "cudaGetDevice"); }
-   if (dev < 0 || dev >= 64) { setError("measure constants: device %d out of range", dev); return MKF_ERR_UNSUPPORTED; }
-   std::lock_guard<std::mutex> lk(gConstMu);
-   if (gConstDone[dev]) { return MKF_OK; }
-   uint8_t member[256];
-   int first[23], n = 0;
-   for (int q = 0; q < 22; q++) {
-      first[q] = n;
-      for (int c = 0; c < 256; c++) {
-         if (kGroupOf[c] == q) { member[n++] = (uint8_t)c; }
-      }
-   }
-   first[22] = n;
-   e = cudaMemcpyToSymbol(cMember, member, sizeof(cMember));
-   if (e == cudaSuccess) { e = cudaMemcpyToSymbol(cFirst, first, sizeof(cFirst)); }
-   if (e == cudaSuccess) { e = cudaMemcpyToSymbol(cWK, kWK, sizeof(cWK)); }
-   if (e == cudaSuccess) { e = cudaMemcpyToSymbol(cWS, kWS, sizeof(cWS)); }
-   if (e == cudaSuccess) { e = cudaMemcpyToSymbol(cWM, kWM, sizeof(cWM)); }
-   if (e != cudaSuccess) { return cudaFail(e, "measure constants upload"); }
-   gConstDone[dev] = true;
-   return MKF_OK;
 }
 
 // Device buffers reused by the host-field path (grown on demand, guarded by a mutex).
@@ -410,8 +369,7 @@ MKF_API int mkfBatchBPFD(uint64_t *pBPFD, const MKFFieldDesc *pF, const MKFThres
 MKF_API int mkfMeasuresF64Dev(double *r, const uint64_t *pBPFD, int nSets, void *stream)
 {
    if (!r || !pBPFD || nSets < 0) { setError("mkfMeasuresF64Dev: bad argument"); return MKF_ERR_ARG; }
-   int rc = uploadConstants();
-   if (rc != MKF_OK || nSets == 0) { return rc; }
+   if (nSets == 0) { return MKF_OK; }
    measuresKernel<<<nSets < 1184 ? nSets : 1184, 128, 0, (cudaStream_t)stream>>>(r, pBPFD, nSets);
    return cudaFail(cudaGetLastError(), "measuresKernel launch");
 }

@@ -369,3 +369,16 @@ for dt, nr in ((np.float32, 4), (np.float64, 2)):
             assert max(c.end - c.begin for c in chunks) > 0
             assert lib.mkfBatchPlanDestroy(h) == 0
 """)
+
+
+def test_measures_on_other_devices_and_after_a_reset(fake):
+    """The measures' tables need no upload, which a reset would undo and a capture would not allow."""
+    fake(r"""
+r, h = np.zeros((3, 4)), np.ones((3, 256), np.uint64)
+for step in (lambda: 0, fake.cudaDeviceReset, lambda: fake.cudaSetDevice(1)):
+    assert step() == 0
+    launches()
+    assert lib.mkfMeasuresF64Dev(r.ctypes.data, h.ctypes.data, 3, None) == 0
+    assert ["measuresKernel" in l[1] for l in launches()] == [True]
+assert fake.fake_calls(b"cudaMemcpyToSymbol") == 0
+""")
