@@ -268,7 +268,7 @@ static int dispatchBallot(const WordTask &a, int enc, cudaStream_t s)
 // Gaussian fields (GRF), plane waves and balls with noise alike, or by more on some than slower on others.
 // B200, time of a call with the other kernel over that with this one, on GRF / waves / balls:
 //  one threshold, word kernel: FP32 64^3 0.87, 128^3 1.07, 256^3 1.07; aligned rows 512^3 0.95, 128 x 2048 x 2048
-//   0.90; other rows 500^3 1.04 / 1.02 / 1.17, 17 x 2048 x 2048 1.32 / 1.24 / 1.40, strided 500^3 1.9; FP64 64^3 0.76,
+//   0.90; other rows 500^3 1.04 / 1.02 / 1.17, 291 x 361 x 823 GRF 0.92, 17 x 2048 x 2048 1.32 / 1.24 / 1.40, strided 500^3 1.9; FP64 64^3 0.76,
 //   128^3 1.04, 256 x 512 x 512 1.13, 333 x 401 x 487 1.31
 //  two to four, word kernel: 100^3 0.7, 128^3 0.9;
 //   strided x: FP32 128^3 0.9, 200 x 210 x 190 0.85 to 1.0, 256^3 1.1 to 1.3, 500^3 1.26 to 1.7; FP64 160 x 150 x 170 0.9
@@ -280,8 +280,8 @@ static int dispatchBallot(const WordTask &a, int enc, cudaStream_t s)
 //   and the votes' 31 cells do not, FP64 512 x 512 x 8 4 thresholds 0.75, 2000 x 1000 x 17 0.6 to 0.8, FP32 512 x 512 x 33 0.7;
 //   few rows: 512 x 6 x 512 FP32 1.1, FP64 1.25 to 1.5; 512 x 40 x 512 FP64 1.03 to 1.15, other rows 1.1 to 1.3;
 //   2000 x 20 x 1000 FP64 aligned 4 thresholds 0.86 / 0.91 / 1.07;
-//   thick fields: FP32 other rows 400^3 2 and 3 thresholds 0.84 / 0.8 / 1.04, 4 1.0 / 1.12 / 1.22 (from 2^26 voxels
-//   on again 0.80 / 1.0 / 1.05, up to 2^27: 599 x 611 x 515 balls 3 thresholds 1.22, 4 1.27, 861 x 841 x 512 5 1.36);
+//   thick fields: FP32 other rows 400^3 2 and 3 thresholds 0.84 / 0.8 / 1.04, 4 1.0 / 1.12 / 1.22, 278 x 222 x 614
+//   GRF 0.89, 500^3 0.80 / 1.0 / 1.05 (from 2^27 voxels on 599 x 611 x 515 balls 3 thresholds 1.22, 4 1.27, 861 x 841 x 512 5 1.36);
 //   FP64 aligned 0.9 to 1.07 but 4 thresholds from 2^24 voxels on 0.97 / 1.06 / 1.07; other rows 2 thresholds
 //   200 x 210 x 190 0.99 / 1.09 / 1.18, 4 0.93 / 1.15 / 1.11, from 2^24 voxels on 1.07 to 1.2
 //  five and six, rank table: strided x FP32 300 x 333 x 277 0.94 / 1.07 / 1.10, 500^3 0.95 / 1.28 / 1.27, FP64 300 x 333 x
@@ -291,7 +291,10 @@ bool useBallots(const WordTask &a, int enc)
 {
    const bool f64 = enc == ENC_F64, aligned = wordRowsAligned(a, enc), strided = a.sx != 1;
    const double voxels = (double)a.X * a.Y * a.Z;
-   if (a.K == 1) { return voxels >= (double)(1 << 20) && (f64 || !aligned || voxels < (double)(1 << 26)); }
+   if (a.K == 1) {
+      return voxels >= (double)(1 << 20) &&
+             (f64 || strided || voxels < (double)(1 << 26) || (!aligned && (a.Z < 34 || voxels >= (double)(1 << 27))));
+   }
    if (a.K > (f64 ? 6 : 5) || voxels < (double)(a.Y < 9 ? 1 << 20 : 1 << 21)) { return false; }
    for (int k = 0; k < a.K && a.K > 2; k++) {  // (two thresholds may differ in their tests)
       if (a.mode[k] != a.mode[0] || a.mode[k] == 3) { return false; }
@@ -315,8 +318,7 @@ bool useBallots(const WordTask &a, int enc)
    }
    if (f64) { return narrow || a.Y < 64 || a.Z < 34 || voxels >= (double)(a.K == 3 ? 1 << 24 : 1 << 22); }
    if (aligned) { return a.Y < 9; }
-   if (narrow || a.Y < (a.K == 4 ? 64 : 16) || a.Z < (voxels < (double)(1 << 23) ? 10 : 34) || voxels >= (double)(1 << 27)) { return true; }
-   return a.K == 4 && voxels >= (double)(1 << 24) && voxels < (double)(1 << 26);
+   return narrow || a.Y < (a.K == 4 ? 64 : 16) || a.Z < (voxels < (double)(1 << 23) ? 10 : 34) || voxels >= (double)(1 << 27);
 }
 
 int launchBallots(WordTask &a, int enc, cudaStream_t s)

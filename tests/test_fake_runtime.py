@@ -264,9 +264,9 @@ F, D = np.float32, np.float64
 table = [
     # one threshold
     (F, (64, 127, 128), "aligned", 1, "word"), (F, (64, 129, 128), "aligned", 1, "vote"), (F, (128, 725, 728), "aligned", 1, "word"),
-    (F, (128, 725, 728), "odd", 1, "vote"), (F, (128, 725, 728), "strided", 1, "vote"), (D, (512, 512, 512), "aligned", 1, "vote"),
+    (F, (128, 725, 728), "odd", 1, "word"), (F, (20, 2000, 2000), "odd", 1, "vote"), (F, (600, 600, 600), "odd", 1, "vote"), (F, (128, 725, 728), "strided", 1, "vote"), (D, (512, 512, 512), "aligned", 1, "vote"),
     # thick fields
-    (F, (300, 300, 300), "aligned", 4, "word"), (F, (300, 300, 300), "odd", 3, "word"), (F, (300, 300, 300), "odd", 4, "vote"), (F, (200, 200, 200), "odd", 4, "word"),
+    (F, (300, 300, 300), "aligned", 4, "word"), (F, (300, 300, 300), "odd", 3, "word"), (F, (300, 300, 300), "odd", 4, "word"), (F, (200, 200, 200), "odd", 4, "word"),
     (F, (500, 500, 500), "odd", 4, "word"), (F, (600, 600, 600), "odd", 3, "vote"), (F, (600, 600, 600), "odd", 5, "vote"),
     (D, (300, 300, 300), "aligned", 3, "word"), (D, (300, 300, 300), "aligned", 4, "vote"), (D, (200, 200, 200), "aligned", 4, "word"),
     (D, (200, 200, 200), "odd", 2, "vote"), (D, (200, 200, 200), "odd", 3, "word"), (D, (300, 300, 300), "odd", 3, "vote"),
