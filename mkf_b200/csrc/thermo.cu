@@ -232,7 +232,14 @@ __global__ void __launch_bounds__(kThWarps * 32, THERMO_MINB) thermoBPFD(const _
 {
    __shared__ ThermoShared S;
    extern __shared__ uint32_t sHist[];
-   ctaSetup<false, (CMAX > 1)>(a, S, sHist);
+   ctaSetup(a, S, sHist);
+   if (CMAX > 1 && a.lutC > kThCandidates) {  // buckets of more thresholds than are compared: the slow path
+      for (int k = threadIdx.x; k + kThCandidates < a.K; k += blockDim.x) {
+         const uint32_t b = S.key[k] >> kLutShift;
+         if (b == S.key[k + kThCandidates] >> kLutShift) { S.lut[b] = kSlowBucket; }
+      }
+      __syncthreads();
+   }
    const long long gw = (long long)blockIdx.x * kThWarps + (threadIdx.x >> 5);
    const long long nw = (long long)gridDim.x * kThWarps;
    unsigned long long cells = 0;

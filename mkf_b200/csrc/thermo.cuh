@@ -217,8 +217,8 @@ __host__ __device__ constexpr size_t thermoDynBytes(int K)
 // Load one field's thresholds, build its rank table and clear the histogram (whole CTA).
 // copyRows: histogram rows per copy (K, or more when rows past K take discarded counts);
 // copies: histogram copies. RAW: the table is indexed by the ranked word's own top bits instead of its
-// order-preserving key's. CROWDED: buckets of more than kThCandidates thresholds take the slow path.
-template <bool RAW = false, bool CROWDED = false, typename P>
+// order-preserving key's.
+template <bool RAW = false, typename P>
 __device__ void ctaSetup(const P &a, ThermoShared &S, uint32_t *hist, int copyRows = 0, int copies = kHistCopies)
 {
    const int K = a.K;
@@ -245,9 +245,8 @@ __device__ void ctaSetup(const P &a, ThermoShared &S, uint32_t *hist, int copyRo
             const int mid = (lo + hi) >> 1;
             if (S.key[mid] < start) { lo = mid + 1; } else { hi = mid; }
          }
-         // (keys < 0x00800000 or >= 0xFF800000, buckets of too many thresholds: the slow path)
-         const bool crowded = CROWDED && lo + kThCandidates < K && (S.key[lo + kThCandidates] >> kLutShift) == b;
-         word |= (b < 32 || b >= kLutSize - 32 || crowded ? kSlowBucket : (uint32_t)lo) << (8 * q);
+         // (keys < 0x00800000 or >= 0xFF800000: the slow path)
+         word |= (b < 32 || b >= kLutSize - 32 ? kSlowBucket : (uint32_t)lo) << (8 * q);
       }
       lut4[w] = word;
    }
