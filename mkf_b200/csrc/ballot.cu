@@ -21,8 +21,9 @@ namespace mkf {
 
 // FP32 fields whose items lie inside the field and are at least kBlPfDepth planes deep load the next
 // plane while counting the current one (two plane buffers in registers at 2 CTAs per SM, 128
-// registers): 1.55 x faster on a 1024^3 FP32 GRF (0.70 vs 1.09 ms), slower for shallow items, which
-// keep the single buffer at 4 CTAs per SM.
+// registers): 1.55 x faster with one threshold on a 1024^3 FP32 GRF (0.70 vs 1.09 ms; fields of that size
+// come here if their rows lie off 16-byte boundaries), slower for shallow items, which keep the single
+// buffer at 4 CTAs per SM.
 static constexpr int kBlPfDepth = 16;
 static constexpr int kBlWarps = 8;
 static constexpr int kBlD = 32;  // default planes of cells per work item

@@ -5,8 +5,9 @@
 // plane by plane and from right to left within a plane. A tile is 32 rows of 128 bytes: 32 elements
 // of a FP32 field, 16 of a FP64 field.
 //  * copy: cp.async fills the warp's ring of tiles in shared memory ahead of the tile it counts, 16
-//    bytes per lane where rows lie on 16-byte boundaries (8 instructions per tile), else one element
-//    per lane; no registers hold data in flight, and the ring runs on over the end of an item into
+//    bytes per lane where rows lie on 16-byte boundaries (8 instructions per tile) and, as the nine
+//    blocks that a row touches, where they lie elsewhere (MIS, 9 instructions); with strided x one
+//    element per lane. No registers hold data in flight, and the ring runs on over the end of an item into
 //    the next;
 //  * map: a lane reads its own row (the 16-byte skew of the row pitch spreads the lanes' 128-bit
 //    reads over all banks) and forms the row's map bits itself, one nibble per element: FP32 as the
