@@ -213,6 +213,9 @@ class BatchPlan:
             descs[i] = _field_desc(f.data_ptr(), _enc_of(f), f.shape, strides)
             sets[i] = self._ths[i].ts
         h = C.c_void_p()
+        # creation counts the batch on a stream of its own: what the current stream still does with the
+        # fields, and with the memory that the counts were allocated from, comes first
+        torch.cuda.current_stream(self.out.device).synchronize()
         check(lib().mkfBatchPlanCreate(C.byref(h), self.out.data_ptr(), descs, sets, n), "mkfBatchPlanCreate")
         self._h = h
 

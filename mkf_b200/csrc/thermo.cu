@@ -492,7 +492,7 @@ int launchThermo(FusedArgs &a, int enc, cudaStream_t s)
    a.lutC = prepareKeys(a, enc);
    // Buckets of more thresholds than the kernel compares send their elements to the exact rank. The word kernel
    // reads the field once for every 8 thresholds instead, which is faster but for many thresholds and larger
-   // fields (B200, us, word kernel / this, thresholds 4 / K around 300 on GRF): 400 x 388 x 416 FP32 17 616 / 729, 24
+   // fields (B200, us, word kernel / this, thresholds 4 / K apart around 300, GRF): 400 x 388 x 416 FP32 17 616 / 729, 24
    // 898 / 1004, 32 1205 / 1126, plane waves 24 758 / 742, 32 1021 / 810, FP64 24 1139 / 1025, 32 1528 / 1150;
    // 2 x 2048 x 2048 FP64 24 169 / 134; 200 x 210 x 190 FP32 24 163 / 182, 32 217 / 216.
    if (a.lutC > kThCandidates && (a.K < 24 || (double)a.X * a.Y * a.Z < (double)(1 << 23))) { return MKF_ERR_UNSUPPORTED; }

@@ -146,3 +146,21 @@ def test_server_shutdown_with_unreleased_counts(mkf, cuda):
     th.start()
     th.join(timeout=60)
     assert done.is_set(), "server shutdown waited for requests that cannot fit"
+
+
+def test_plan_creation_waits_for_the_current_stream(mkf, cuda):
+    """A plan's creation counts the batch on its own stream; the counts' memory may have been in use by work
+    that the current stream has not done yet."""
+    import torch
+
+    f = torch.randn((40, 40, 40), device=cuda)
+    x = torch.full((4, 256), 7, dtype=torch.int64, device=cuda)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)
+    y = x.clone()
+    g = torch.randn((40, 40, 40), device=cuda)
+    del x  # (its block goes to the plan's counts)
+    p = mkf.BatchPlan([f, g], [[0.0, 0.5], [0.0, 0.5]])
+    assert (y == 7).all()
+    assert torch.equal(p.launch(), torch.cat([mkf.field_bpfd(f, [0.0, 0.5]), mkf.field_bpfd(g, [0.0, 0.5])]))
+    p.close()
