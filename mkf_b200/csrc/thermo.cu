@@ -1,6 +1,7 @@
 // thermo.cu - fused counting kernel for threshold sets that share one relation (< <= > >=), reading
 // the field straight from global memory: 17 to 32 thresholds, fields too small for the staged
-// kernel's tiles (thermo_tma.cu), and the small fields of a batch with more than kWordMaxK thresholds.
+// kernel's tiles (thermo_tma.cu), large FP64 fields with strided x, and the small fields of a batch with
+// more than kWordMaxK thresholds or of one that needs no word kernel (BatchMix).
 //
 // Sorted thresholds make an element's K map bits a thermometer, bits[k] = (k < rank), so an
 // element reduces to one rank 0..K. The rank is found with a table over order-preserving 32-bit
@@ -9,7 +10,7 @@
 // four when thresholds share a bucket) finishes the count. FP32 keys are exact. A FP64 element is
 // read as its high word only (same DRAM sectors, half the load bandwidth into the SM); when that
 // word ties with the candidate's, the element is re-read whole and ranked exactly by binary
-// search. Infinities and NaNs (and FP64 magnitudes of 2^1017 and more) fall in table buckets
+// search, as are the elements of a bucket that more than four thresholds share. Infinities and NaNs (and FP64 magnitudes of 2^1017 and more) fall in table buckets
 // flagged for the same exact path.
 //
 // A warp owns 32 x positions (31 cells, neighbouring columns overlap by one element), TY row pairs
